@@ -126,6 +126,12 @@ int shield_mp_create(const ShieldMpConfig* cfg, int nx, int ny, int nz, ShieldFi
  * differs from the previous one recomputes the sub-step (_set_timestep). */
 int shield_mp_step(void* handle, const ShieldMpFields* fields, double timestep, int precision, void* stream);
 
+/* shield_mp_step in the plain form with the rounding of every operation of
+ * the reference's expressions (CUDA's exp, log and pow, IEEE division): the
+ * forward step of a differentiated window, whose branches may hang on the
+ * sign of a rounding residue. Agrees with shield_mp_step to round-off. */
+int shield_mp_step_ieee(void* handle, const ShieldMpFields* fields, double timestep, void* stream);
+
 int shield_mp_destroy(void* handle);
 
 /* Copies the handle's last error message (NUL terminated) into buf. */

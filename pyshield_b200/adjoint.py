@@ -29,7 +29,6 @@ import ctypes
 from ._lib import (
     MP_STATE_FIELDS,
     MP_TENDENCY_FIELDS,
-    SHIELD_MP_PLAIN,
     ShieldMpCotangents,
     ShieldMpFields,
     ShieldMpGradients,
@@ -105,9 +104,11 @@ def step_forward(mp, state, land, timestep, stream=None, tendencies=None):
     pr = torch.zeros((4, mp.ny, mp.nx), dtype=torch.float64, device=state[0].device)
     base, plane = pr.data_ptr(), mp.nx * mp.ny * 8
     F.rain, F.snow, F.ice, F.graupel = base, base + plane, base + 2 * plane, base + 3 * plane
-    rc = load().shield_mp_step(mp._handle, ctypes.byref(F), float(timestep), SHIELD_MP_PLAIN,
-                               ctypes.c_void_p(_current_stream(stream)))
-    check(rc, mp._handle, "shield_mp_step")
+    # the form that keeps the reference's rounding: a window's branches may
+    # hang on the sign of a rounding residue (csrc/mp_ieee.cu)
+    rc = load().shield_mp_step_ieee(mp._handle, ctypes.byref(F), float(timestep),
+                                    ctypes.c_void_p(_current_stream(stream)))
+    check(rc, mp._handle, "shield_mp_step_ieee")
     qaz = mp.get_qaz().permute(2, 1, 0)
     return tuple(tend) + (w_out, qaz) + tuple(pr[i].t() for i in range(4))
 

@@ -19,9 +19,10 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 BUILD = os.path.join(HERE, "_build")
 LIB = os.path.join(HERE, "libshield_mp.so")
-# the FP64 throughput probe bench.py uses for the step kernel's FP64 roofline
-# (not part of the C-ABI)
+# the FP64 throughput probe bench.py uses for the step kernel's FP64 roofline,
+# and the device math the tests measure (not part of the C-ABI)
 PROBE_LIB = os.path.join(HERE, "libshield_probe.so")
+PROBE_UNITS = ("peak.cu", "math_probe.cu")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 COMMON = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-Xcompiler", "-ffp-contract=off",
           "--expt-relaxed-constexpr", "-I", os.path.join(os.path.dirname(HERE), "include")]
@@ -30,6 +31,7 @@ COMMON = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-Xcompiler",
 UNITS = [
     ("capi.cu", ["-fmad=false"]),
     ("mp_plain.cu", ["-fmad=false"]),
+    ("mp_ieee.cu", ["-fmad=false"]),
     # the mixed form's FP32 process rates use the hardware's approximate
     # exp2 / log2 / reciprocal / square root with denormals flushed (these
     # options act on single precision only; its FP64 is unchanged)
@@ -61,19 +63,20 @@ def _stale(objs):
     if not os.path.exists(LIB):
         return True
     t = os.path.getmtime(LIB)
-    deps = [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f != "peak.cu"] + [os.path.join(os.path.dirname(HERE), "include", "shield_mp.h"), __file__]
+    deps = [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f not in PROBE_UNITS] + [os.path.join(os.path.dirname(HERE), "include", "shield_mp.h"), __file__]
     return any(os.path.getmtime(d) > t for d in deps if os.path.exists(d))
 
 
 def build(force=False, jobs=None, verbose=False):
     units = [u for u in UNITS if os.path.exists(os.path.join(CSRC, u[0]))]
-    probe_src = os.path.join(CSRC, "peak.cu")
-    if force or not os.path.exists(PROBE_LIB) or os.path.getmtime(probe_src) > os.path.getmtime(PROBE_LIB):
+    probe_src = [os.path.join(CSRC, f) for f in PROBE_UNITS]
+    probe_deps = probe_src + [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".cuh", ".h"))]
+    if force or not os.path.exists(PROBE_LIB) or max(map(os.path.getmtime, probe_deps)) > os.path.getmtime(PROBE_LIB):
         tmp = PROBE_LIB + ".tmp"
-        r = subprocess.run([nvcc()] + ARCH + COMMON + ["-shared", "-o", tmp, probe_src, "-cudart", "static"],
-                           capture_output=True, text=True)
+        r = subprocess.run([nvcc()] + ARCH + COMMON + ["-fmad=false", "-shared", "-o", tmp] + probe_src
+                           + ["-cudart", "static"], capture_output=True, text=True)
         if r.returncode != 0:
-            raise RuntimeError(f"nvcc failed for peak.cu:\n{r.stdout}\n{r.stderr}")
+            raise RuntimeError(f"nvcc failed for the probes:\n{r.stdout}\n{r.stderr}")
         os.replace(tmp, PROBE_LIB)
     if not force and not _stale(units):
         return LIB

@@ -108,9 +108,10 @@ extern "C" int shield_mp_create(const ShieldMpConfig* cfg, int nx, int ny, int n
 namespace {
 
 // The step of shield_mp_step; with `flags` non-null (plain form only) the
-// launch also records each sub-step's column flags there.
+// launch also records each sub-step's column flags there; with `ieee` (plain
+// form only) it keeps the reference's rounding.
 int step_impl(Handle* h, const ShieldMpFields* F, double timestep, int precision, int32_t* flags, int64_t nflags,
-              void* stream) {
+              void* stream, bool ieee = false) {
   if (!h) return fail(nullptr, SHIELD_EINVAL, "null handle");
   if (!F) return fail(h, SHIELD_EINVAL, "null fields");
   if (precision != SHIELD_MP_PLAIN && precision != SHIELD_MP_MIXED)
@@ -167,7 +168,7 @@ int step_impl(Handle* h, const ShieldMpFields* F, double timestep, int precision
     e = mp_launch_de_ice(A, f3(F->qi_dt), f3(F->qs_dt), st);
     if (e != cudaSuccess) return cuda_fail(h, e, "de_ice launch");
   }
-  e = flags ? mp_launch_plain_flags(A, st) : mp_launch_step(A, precision, st);
+  e = flags ? mp_launch_plain_flags(A, st) : ieee ? mp_launch_ieee(A, st) : mp_launch_step(A, precision, st);
   if (e != cudaSuccess) return cuda_fail(h, e, "microphysics launch");
   return SHIELD_OK;
 }
@@ -176,6 +177,10 @@ int step_impl(Handle* h, const ShieldMpFields* F, double timestep, int precision
 
 extern "C" int shield_mp_step(void* handle, const ShieldMpFields* F, double timestep, int precision, void* stream) {
   return step_impl(static_cast<Handle*>(handle), F, timestep, precision, nullptr, 0, stream);
+}
+
+extern "C" int shield_mp_step_ieee(void* handle, const ShieldMpFields* F, double timestep, void* stream) {
+  return step_impl(static_cast<Handle*>(handle), F, timestep, SHIELD_MP_PLAIN, nullptr, 0, stream, true);
 }
 
 extern "C" int shield_mp_step_flags(void* handle, const ShieldMpFields* F, double timestep, int32_t* flags,

@@ -1,0 +1,51 @@
+// The device math of mp_math.cuh and the saturation humidity built on it,
+// one call per element, for the tests that measure their errors. Part of the
+// probe library, not of the C-ABI.
+#include <cuda_runtime.h>
+
+#include <cstring>
+
+#include "mp_physics.cuh"
+#include "mp_setup.h"
+
+namespace {
+
+using namespace shield;
+
+enum { F_DIV = 0, F_SQRT, F_EXP, F_LOG, F_POW, F_QSW, F_QSW_DT, F_QSI, F_QSI_DT };
+
+__global__ void math_kernel(int fn, int n, const double* x, const double* y, double* out,
+                            const __grid_constant__ MpConst K) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const double a = x[i], b = y[i];
+  double r = 0.0, d = 0.0;
+  switch (fn) {
+    case F_DIV: r = qdiv(a, b); break;
+    case F_SQRT: r = qsqrt(a); break;
+    case F_EXP: r = xexp(a); break;
+    case F_LOG: r = xlog(a); break;
+    case F_POW: r = xpowc(a, b); break;
+    case F_QSW: r = wqs1(K, a, b); break;
+    case F_QSW_DT: wqs2(K, a, b, d), r = d; break;
+    case F_QSI: r = iqs1(K, a, b); break;
+    case F_QSI_DT: iqs2(K, a, b, d), r = d; break;
+  }
+  out[i] = r;
+}
+
+}  // namespace
+
+// out[i] = function `fn` of (x[i], y[i]) for n elements on `stream`: a / b,
+// sqrt, exp, log, x^y, then wqs1, its derivative, iqs1, its derivative at
+// temperature x and density y.
+extern "C" int shield_probe_math(int fn, int n, const double* x, const double* y, double* out, void* stream) {
+  if (fn < F_DIV || fn > F_QSI_DT || n < 1 || !x || !y || !out) return -1;
+  ShieldMpConfig cfg;
+  std::memset(&cfg, 0, sizeof(cfg));
+  MpConst K;
+  std::memset(&K, 0, sizeof(K));
+  setupm(cfg, K);
+  math_kernel<<<(n + 255) / 256, 256, 0, static_cast<cudaStream_t>(stream)>>>(fn, n, x, y, out, K);
+  return cudaGetLastError() == cudaSuccess ? 0 : -3;
+}

@@ -28,6 +28,7 @@
 #include "mp_physics_mixed.cuh"
 
 namespace shield {
+inline namespace SHIELD_ARITH {
 
 #define FULLMASK 0xffffffffu
 
@@ -749,15 +750,15 @@ SHD double implicit_fall(Col& C, double& q, double vt, double dz, double dp1, bo
   const double dd = dtf * vt;
   const double qmass = valid ? q * dp1 : 0.0;
   const double ddp = C.prev(dd);
-  const double D = dz + dd;
-  double a = qmass / D;
-  double b = (C.k == 0) ? 0.0 : ddp / D;
+  const Divisor<double> by_D(dz + dd);
+  double a = by_D(qmass);
+  double b = (C.k == 0) ? 0.0 : by_D(ddp);
   if (!valid) {
     a = 0.0;
     b = 0.0;
   }
   const double r = C.scan_affine(a, b);
-  if (valid) q = r * dz / dp1;
+  if (valid) q = qdiv(r * dz, dp1);
   return valid ? dd * r : 0.0;
 }
 
@@ -771,12 +772,12 @@ SHD void sedi_heat(Col& C, const MpConst& K, double& tz, double dz1, double dp1,
   double a, b;
   if (C.k == 0) {
     const double tmp = cvn + flux * c_cond;
-    a = tz + flux * dgz / tmp;
+    a = tz + qdiv(flux * dgz, tmp);
     b = 0.0;
   } else {
-    const double D = cvn + c_cond * flux;
-    a = ((cvn + c_cond * (flux - fp)) * tz + dgz * (fp + flux)) / D;
-    b = fp * c_cond / D;
+    const Divisor<double> by_D(cvn + c_cond * flux);
+    a = by_D((cvn + c_cond * (flux - fp)) * tz + dgz * (fp + flux));
+    b = by_D(fp * c_cond);
   }
   if (!valid) {
     a = tz;
@@ -788,8 +789,8 @@ SHD void sedi_heat(Col& C, const MpConst& K, double& tz, double dz1, double dp1,
 // Vertical-velocity update by one falling species given the flux and fall
 // speed at this level and the level above (microphysics.py:492-515).
 SHD double w_update(int k, double w, double dm, double flux, double vt, double fp, double vp) {
-  if (k == 0) return (dm * w + flux * vt) / (dm - flux);
-  return (dm * w - fp * vp + flux * vt) / (dm + fp - flux);
+  if (k == 0) return qdiv(dm * w + flux * vt, dm - flux);
+  return qdiv(dm * w - fp * vp + flux * vt, dm + fp - flux);
 }
 
 // Monotone vertical slope for autoconversion (microphysics.py:595-620,
@@ -802,10 +803,10 @@ SHD double mono_slope(Col& C, double q) {
   const double dqn = 0.5 * (qn - q);
   double v = 0.0;
   if (C.k >= 1 && C.k <= C.L - 2) {
-    v = 0.5 * fmin(fabs(dq + dqn), 0.5 * q);
+    v = 0.5 * qmin(fabs(dq + dqn), 0.5 * q);
     if (dq * dqn <= 0.0) {
       if (dq > 0.0)
-        v = fmin(v, fmin(dq, -dqn));
+        v = qmin(v, qmin(dq, -dqn));
       else
         v = 0.0;
     }
@@ -993,14 +994,14 @@ SHD void fields_init(Col& C, const MpConst& K, bool valid, double pt, double qvi
   S.tz = pt;
   P.dp1 = delp;
   P.dp1 = P.dp1 * (1.0 - qvi);
-  const double omq = delp / P.dp1;
+  const double omq = qdiv(delp, P.dp1);
   S.qv = qvi * omq;
   S.ql = qli * omq;
   S.qr = qri * omq;
   S.qi = qii * omq;
   S.qs = qsi * omq;
   S.qg = qgi * omq;
-  const double den0 = -P.dp1 / (K.GRAV * dz0);
+  const double den0 = qdiv(-P.dp1, K.GRAV * dz0);
   P.p1 = den0 * K.RDGAS * pt;
   S.w = wz;
   double ccn;
@@ -1011,18 +1012,18 @@ SHD void fields_init(Col& C, const MpConst& K, bool valid, double pt, double qvi
     if (K.use_ccn) {
       double tzb, p1b;
       C.bcast2(S.tz, P.p1, L - 1, tzb, p1b);
-      ccn = ccn * K.RDGAS * tzb / p1b;
+      ccn = qdiv(ccn * K.RDGAS * tzb, p1b);
     }
   }
   P.ccn = ccn;
-  P.c_praut = K.cpaut * xpow(ccn * RHOR, -1.0 / 3.0);
-  const double s_leng = sqrt(sqrt(area * 1.0e-10));
+  P.c_praut = K.cpaut * xpowp(ccn * RHOR, -1.0 / 3.0);
+  const double s_leng = qsqrt(qsqrt(area * 1.0e-10));
   const double t_land = K.dw_land * s_leng;
   const double t_ocean = K.dw_ocean * s_leng;
   double h_var = t_land * land + t_ocean * (1.0 - land);
-  P.h_var = fmin(0.2, fmax(0.01, h_var));
+  P.h_var = qmin(0.2, qmax(0.01, h_var));
   P.rh_adj = 1.0 - P.h_var - K.rh_inc;
-  P.rh_rain = fmax(0.35, P.rh_adj - K.rh_inr);
+  P.rh_rain = qmax(0.35, P.rh_adj - K.rh_inr);
 
   if (K.fix_negative) {
     fix_negative_point(K, S.qv, S.ql, S.qr, S.qi, S.qs, S.qg, S.tz);
@@ -1053,9 +1054,9 @@ SHD void fields_init(Col& C, const MpConst& K, bool valid, double pt, double qvi
     C.bcast2(S.qv, P.dp1, L - 1, qb, db);
     C.bcast2(S.qv, P.dp1, L - 2, qb1, db1);
     if ((qb < 0.0) && (qb1 > 0.0)) {
-      const double dq = fmin(-qb * db, qb1 * db1);
-      if (k == L - 2) S.qv = S.qv - dq / P.dp1;
-      if (k == L - 1) S.qv = S.qv + dq / P.dp1;
+      const double dq = qmin(-qb * db, qb1 * db1);
+      if (k == L - 2) S.qv = S.qv - qdiv(dq, P.dp1);
+      if (k == L - 1) S.qv = S.qv + qdiv(dq, P.dp1);
     }
   }
 }
@@ -1065,10 +1066,10 @@ SHD void fields_init(Col& C, const MpConst& K, bool valid, double pt, double qvi
 template <class Col>
 SHD void substep_geometry(Col& C, const MpConst& K, bool valid, double t0, double dz0, const LevState& S,
                           StepGeom& P) {
-  const double den0 = -P.dp1 / (K.GRAV * dz0);
-  P.dz1 = dz0 * S.tz / t0;
-  P.den = den0 * dz0 / P.dz1;
-  P.denfac = sqrt(SFCRHO / P.den);
+  const double den0 = qdiv(-P.dp1, K.GRAV * dz0);
+  P.dz1 = qdiv(dz0 * S.tz, t0);
+  P.den = qdiv(den0 * dz0, P.dz1);
+  P.denfac = qsqrt(qdiv(SFCRHO, P.den));
   P.dz = C.heights(valid ? -P.dz1 : 0.0, K.zs);
 }
 
@@ -1146,9 +1147,9 @@ SHD void warm_rain(Col& C, const MpConst& K, const MpConstF& KF, bool valid, Lev
     if (K.z_slope_liq) {
       dl = mono_slope(C, ql);
       rec.value(0, dl);
-      dl = fmax(dl, fmax(QVMIN, P.h_var * ql));
+      dl = qmax(dl, qmax(QVMIN, P.h_var * ql));
     } else {
-      dl = fmax(QVMIN, P.h_var * ql);
+      dl = qmax(QVMIN, P.h_var * ql);
     }
     if constexpr (MIXED)
       autoconv_subgrid_var_m(K, KF, ql, qr, tz, P.den, P.ccn, P.c_praut, dl);
@@ -1202,9 +1203,9 @@ SHD void sedimentation(Col& C, const MpConst& K, const MpConstF& KF, bool valid,
 #pragma unroll
     for (int n = 0; n < 3; ++n) {
       const double qmass = valid ? qq[n] * dp1 : 0.0;
-      const double D = dz + dd[n];
-      ra[n] = qmass / D;
-      rb[n] = (k == 0) ? 0.0 : ddp[n] / D;
+      const Divisor<double> by_D(dz + dd[n]);
+      ra[n] = by_D(qmass);
+      rb[n] = (k == 0) ? 0.0 : by_D(ddp[n]);
       if (!valid) {
         ra[n] = 0.0;
         rb[n] = 0.0;
@@ -1214,12 +1215,13 @@ SHD void sedimentation(Col& C, const MpConst& K, const MpConstF& KF, bool valid,
     double flux[3];
 #pragma unroll
     for (int n = 0; n < 3; ++n) flux[n] = valid ? dd[n] * r[n] : 0.0;
+    const Divisor<double> by_dp1(dp1);
     const double dm_i = dp1 * (1.0 + qv + ql + qr + qi + qs + qg);
-    if (fi && valid) qi = r[0] * dz / dp1;
+    if (fi && valid) qi = by_dp1(r[0] * dz);
     const double dm_s = dp1 * (1.0 + qv + ql + qr + qi + qs + qg);
-    if (fs && valid) qs = r[1] * dz / dp1;
+    if (fs && valid) qs = by_dp1(r[1] * dz);
     const double dm_g = dp1 * (1.0 + qv + ql + qr + qi + qs + qg);
-    if (fg && valid) qg = r[2] * dz / dp1;
+    if (fg && valid) qg = by_dp1(r[2] * dz);
     double sfc[3];
     C.template bcastN<3>(flux, L - 1, sfc);
     const double nv[6] = {flux[0], vti, flux[1], vts, flux[2], vtg};
@@ -1262,9 +1264,9 @@ SHD void icloud(Col& C, const MpConst& K, const MpConstF& KF, bool valid, LevSta
   if (K.z_slope_ice) {
     di = mono_slope(C, qi);
     rec.value(0, di);
-    di = fmax(di, fmax(QVMIN, P.h_var * qi));
+    di = qmax(di, qmax(QVMIN, P.h_var * qi));
   } else {
-    di = fmax(QVMIN, P.h_var * qi);
+    di = qmax(QVMIN, P.h_var * qi);
   }
   if (valid) {
     if constexpr (MIXED)
@@ -1363,20 +1365,20 @@ SHD void mp_body(const MpArgs& A, double* sm, double* scr, double* work, const i
       av = v0;
       b = 0.0;
     } else {
-      const double D = dp0 + mp;
-      au = dp0 * u0 / D;
-      av = dp0 * v0 / D;
-      b = mp / D;
+      const Divisor<double> by_D(dp0 + mp);
+      au = by_D(dp0 * u0);
+      av = by_D(dp0 * v0);
+      b = by_D(mp);
     }
     C.scan_affine2(au, b, av, b, u1, v1);
   }
   if (valid) {
     const double rdt = K.rdt;
-    const double omq0 = dp0 / dp1;
+    const double omq0 = qdiv(dp0, dp1);
     const double qv0 = TL(IN_QV) * omq0, ql0 = TL(IN_QL) * omq0, qr0 = TL(IN_QR) * omq0;
     const double qi0 = TL(IN_QI) * omq0, qs0 = TL(IN_QS) * omq0, qg0 = TL(IN_QG) * omq0;
     const double t0 = TL(IN_PT), qa0 = TL(IN_QA);
-    const double omq = dp1 / dp0;
+    const double omq = qdiv(dp1, dp0);
     const double inc_qv = rdt * (qv - qv0) * omq;
     const double inc_ql = rdt * (ql - ql0) * omq;
     const double inc_qr = rdt * (qr - qr0) * omq;
@@ -1384,8 +1386,8 @@ SHD void mp_body(const MpArgs& A, double* sm, double* scr, double* work, const i
     const double inc_qs = rdt * (qs - qs0) * omq;
     const double inc_qg = rdt * (qg - qg0) * omq;
     const double cvm = K.c_air + qv * K.c_vap + (qr + ql) * K.C_LIQ + (qi + qs + qg) * K.C_ICE;
-    const double inc_pt = rdt * (tz - t0) * cvm / K.CP_AIR;
-    const double inc_qa = K.do_qa ? 0.0 : rdt * (qa / (double)K.ntimes - qa0);
+    const double inc_pt = qdivc(rdt * (tz - t0) * cvm, PH_CP_AIR, 1.0 / PH_CP_AIR);
+    const double inc_qa = K.do_qa ? 0.0 : rdt * (qdiv(qa, (double)K.ntimes) - qa0);
     const double inc_u = K.sedi_transport ? (u1 - u0) * rdt : 0.0;
     const double inc_v = K.sedi_transport ? (v1 - v0) * rdt : 0.0;
     TL(OUT_PT_DT) = inc_pt;
@@ -1664,6 +1666,37 @@ using Packed80 = PackedLayout<SHIELD_PACK_NWG, SHIELD_PACK_P, SHIELD_PACK_NGRP>;
 constexpr int PACK80_MINB = SHIELD_PACK_MINB;
 constexpr int PACK80_LMIN = 65, PACK80_LMAX = 80;
 
+// Launch shape for 81-96 levels: columns per block and the minimum resident
+// blocks per SM given to __launch_bounds__ (which caps the registers per
+// thread). Four columns per block (one 384-thread block per SM) measured
+// fastest: the staging then reads whole 32-byte sectors. 65-80 levels (L79)
+// pack two columns per 5 warps (Packed80).
+#ifndef SHIELD_NW3_G
+#define SHIELD_NW3_G 4
+#endif
+#ifndef SHIELD_NW3_MINB
+#define SHIELD_NW3_MINB 1
+#endif
+// 97..128 levels (L127): columns per block of 4 warps each. C96 L127 (ms):
+// 4 columns (512 threads, 128 registers) 6.29, 5 columns (640, 96) 5.94,
+// 6 columns (768, 80) 5.99.
+#ifndef SHIELD_NW4_G
+#define SHIELD_NW4_G 5
+#endif
+
+// The plain form's launch for each level range (FLAGS: with the column flags
+// recorded).
+template <bool FLAGS>
+cudaError_t launch_plain_shapes(const MpArgs& A, cudaStream_t st) {
+  const int L = A.nz;
+  if (L <= 32) return launch_step<ColumnLayout<1, 4>, 2, false, false, FLAGS>(A, st);
+  if (L <= 64) return launch_step<ColumnLayout<2, 2>, 2, false, false, FLAGS>(A, st);
+  if (L <= PACK80_LMAX) return launch_step<Packed80, PACK80_MINB, false, false, FLAGS>(A, st);
+  if (L <= 96) return launch_step<ColumnLayout<3, SHIELD_NW3_G>, SHIELD_NW3_MINB, false, false, FLAGS>(A, st);
+  if (L <= 128) return launch_step<ColumnLayout<4, SHIELD_NW4_G>, 1, false, false, FLAGS>(A, st);
+  return launch_step<ColumnLayout<8, 1>, 2, false, false, FLAGS>(A, st);
+}
+
 // Launch of the ensemble kernel with `grid` persistent blocks; `counter`
 // (one word) is zeroed on `st` first.
 template <class LY, int MINB, bool MIXED>
@@ -1678,4 +1711,5 @@ cudaError_t launch_ensemble(const MpArgs* members, const int64_t* offs, int nm, 
   return cudaGetLastError();
 }
 
+}  // namespace SHIELD_ARITH
 }  // namespace shield

@@ -3,7 +3,24 @@
 
 #include <cstdint>
 
+// The device code of a unit that keeps IEEE rounding (SHIELD_IEEE, see
+// mp_math.cuh) lives in a namespace of its own.
+#ifdef SHIELD_IEEE
+#define SHIELD_ARITH ieee
+#else
+#define SHIELD_ARITH quick
+#endif
+
 namespace shield {
+
+// The physical constants (pyshield_b200/constants.py), for the functions that
+// want them as literals; setupm copies them into MpConst.
+constexpr double PH_RVGAS = 461.50, PH_C_ICE = 1972.0, PH_C_LIQ = 4.1855e3, PH_TICE = 273.16, PH_E00 = 611.21;
+constexpr double PH_HLV = 2.5e6, PH_HLF = 3.3358e5, PH_CP_AIR = 1004.6;
+constexpr double PH_DC_VAP = 4.0 * PH_RVGAS - PH_C_LIQ, PH_DC_ICE = PH_C_LIQ - PH_C_ICE;
+constexpr double PH_D2ICE = PH_DC_VAP + PH_DC_ICE;
+constexpr double PH_LV0 = PH_HLV - PH_DC_VAP * PH_TICE, PH_LI00 = PH_HLF - PH_DC_ICE * PH_TICE;
+constexpr double PH_LI2 = PH_LV0 + PH_LI00;
 
 // Every scalar the step reads: the physical constants, the process constants
 // of Microphysics.setupm (pySHiELD/stencils/microphysics.py:1813-1953), the
@@ -27,12 +44,11 @@ struct MpConst {
       rh_inr, vi_fac, vs_fac, vg_fac, vr_fac, vi_max, vs_max, vg_max, vr_max, ccn_l, ccn_o;
   int do_qa, const_vg, const_vi, const_vr, const_vs, rad_snow, rad_rain, do_sedi_heat, do_sedi_w, fast_sat_adj,
       fix_negative, irain_f, prog_ccn, use_ccn, sedi_transport, z_slope_ice, z_slope_liq, de_ice;
+  double r_log_10;  // 1 / log_10
 };
 
 // FP32 copies of the constants the mixed form's process rates use.
 struct MpConstF {
-  // FP64 constants of the mixed form's saturation adjustment (qsat_m)
-  double qs_e00, qw_c1, qw_c2, qw_c3, qi_c1, qi_c2, qi_c3, qs_t0, qs_tmin, qs_thi, qi_lo, qi_lo_dq;
   double qs_rtw;  // 1 / (tice - t_wfr) of the saturation adjustment
   float E00, DC_VAP, LV0, D2ICE, LI2, RVGAS, TICE, T_SAT_MIN, iqs_lo_num, LAT2;
   float cracs, csacr, cgacr, cgacs, acco[3][4], csacw, csaci, cgacw, cgaci, cracw, cssub[5], crevp[5], cgfr[2],

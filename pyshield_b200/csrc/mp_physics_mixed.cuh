@@ -18,6 +18,7 @@
 #include "mp_physics.cuh"
 
 namespace shield {
+inline namespace SHIELD_ARITH {
 
 SHD float sqf(float x) { return x * x; }
 SHD float dimf(float x, float y) {
@@ -52,14 +53,14 @@ SHD void revap_racc_m(const MpConst& K, const MpConstF& F, double dt, double h_v
     double q_liq = ql + qr;
     const double q_sol = qi + qs + qg;
     double cvm = cvm_of(K, qv, q_liq, q_sol);
-    const double lcpk = lhl / cvm;
+    const double lcpk = qdiv(lhl, cvm);
     const double tin = tz - lcpk * ql;
     const double qpz = qv + ql;
     float dqsdt_f;
     const double qsat = wqs2_f(F, (float)tin, (float)den, dqsdt_f);
     const double dqsdt = dqsdt_f;
-    double dqh = fmax(ql, h_var * fmax(qpz, QCMIN));
-    dqh = fmin(dqh, 0.2 * qpz);
+    double dqh = qmax(ql, h_var * qmax(qpz, QCMIN));
+    dqh = qmin(dqh, 0.2 * qpz);
     const double dqv = qsat - qv;
     const double q_minus = qpz - dqh;
     const double q_plus = qpz + dqh;
@@ -73,12 +74,12 @@ SHD void revap_racc_m(const MpConst& K, const MpConstF& F, double dt, double h_v
       const float t2 = (float)tin * (float)tin;
       const float evap_rate = F.crevp[0] * t2 * dq * (F.crevp[1] * sqrtf(qden) + F.crevp[2] * expf(0.725f * logf(qden))) /
                               (F.crevp[3] * t2 + F.crevp[4] * (float)qsat * (float)den);
-      const double evap = fmin(qr, fmin(dt * (double)evap_rate, dqv / (1.0 + lcpk * dqsdt)));
+      const double evap = qmin(qr, qmin(dt * (double)evap_rate, qdiv(dqv, 1.0 + lcpk * dqsdt)));
       qr = qr - evap;
       qv = qv + evap;
       q_liq = q_liq - evap;
       cvm = cvm_of(K, qv, q_liq, q_sol);
-      tz = tz - evap * lhl / cvm;
+      tz = tz - qdiv(evap * lhl, cvm);
     }
     if ((qr > QRMIN) && (ql > 1.0e-6) && (qsat < q_minus)) {
       float sink = (float)dt * (float)denfac * F.cracw * expf(0.95f * logf((float)(qr * den)));
@@ -105,7 +106,7 @@ SHD void fall_speed_m(const MpConst& K, const MpConstF& F, double qg, double qi,
     float v = (3.0f + logf((float)qi * denf) / F.log_10) * (tc * ((float)AA * tc + (float)BB) + (float)CC) +
               (float)DD_FS * tc + (float)EE;
     v = vi0 * expf(F.log_10 * v) * 0.8f;
-    vti = fmin(K.vi_max, fmax(VF_MIN, (double)v));
+    vti = qmin(K.vi_max, qmax(VF_MIN, (double)v));
   }
   if (K.const_vs) {
     vts = K.vs_fac;
@@ -113,7 +114,7 @@ SHD void fall_speed_m(const MpConst& K, const MpConstF& F, double qg, double qi,
     vts = VF_MIN;
   } else {
     const float v = (float)K.vs_fac * (float)VCONS * rhof * expf(0.0625f * logf((float)qs * denf / (float)NORMS));
-    vts = fmin(K.vs_max, fmax(VF_MIN, (double)v));
+    vts = qmin(K.vs_max, qmax(VF_MIN, (double)v));
   }
   if (K.const_vg) {
     vtg = K.vg_fac;
@@ -121,7 +122,7 @@ SHD void fall_speed_m(const MpConst& K, const MpConstF& F, double qg, double qi,
     vtg = VF_MIN;
   } else {
     const float v = (float)K.vg_fac * (float)VCONG * rhof * sqrtf(sqrtf(sqrtf((float)qg * denf / (float)NORMG)));
-    vtg = fmin(K.vg_max, fmax(VF_MIN, (double)v));
+    vtg = qmin(K.vg_max, qmax(VF_MIN, (double)v));
   }
 }
 
@@ -131,7 +132,7 @@ SHD double rain_fspeed_m(const MpConst& K, double qrz, double den) {
   const float denf = (float)den;
   const float v = (float)K.vr_fac * (float)VCONR * sqrtf(fminf(10.0f, (float)SFCRHO / denf)) *
                   expf(0.2f * logf((float)qrz * denf / (float)NORMR));
-  return fmin(K.vr_max, fmax(VR_MIN, (double)v));
+  return qmin(K.vr_max, qmax(VR_MIN, (double)v));
 }
 
 // ---------------------------------------------------- microphysics_funcs.py:375-428
@@ -139,11 +140,11 @@ SHD void autoconv_no_subgrid_var_m(const MpConst& K, const MpConstF& F, double& 
                                    double den, double ccn, double c_praut) {
   const double qc0 = K.fac_rc * ccn;
   if (tz > K.t_wfr) {
-    const double qc = K.use_ccn ? qc0 : qc0 / den;
+    const double qc = K.use_ccn ? qc0 : qdiv(qc0, den);
     const double dq = qlz - qc;
     if (dq > 0.0) {
       const float rate = F.dt_rain * (float)c_praut * (float)den * expf(F.so3 * logf((float)qlz));
-      const double sink = fmin(dq, (double)rate);
+      const double sink = qmin(dq, (double)rate);
       qlz = qlz - sink;
       qrz = qrz + sink;
     }
@@ -153,11 +154,11 @@ SHD void autoconv_subgrid_var_m(const MpConst& K, const MpConstF& F, double& qlz
                                 double ccn, double c_praut, double dl) {
   const double qc0 = K.fac_rc * ccn;
   if (tz > K.t_wfr + DT_FR) {
-    dl = fmin(fmax(1.0e-6, dl), 0.5 * qlz);
-    const double qc = K.use_ccn ? qc0 : qc0 / den;
+    dl = qmin(qmax(1.0e-6, dl), 0.5 * qlz);
+    const double qc = K.use_ccn ? qc0 : qdiv(qc0, den);
     const double dq = 0.5 * (qlz + dl - qc);
     if (dq > 0.0) {
-      const float rate = fminf(1.0f, (float)(dq / dl)) * F.dt_rain * (float)c_praut * (float)den *
+      const float rate = fminf(1.0f, (float)qdiv(dq, dl)) * F.dt_rain * (float)c_praut * (float)den *
                          expf(F.so3 * logf((float)qlz));
       const double sink = (double)rate;
       qlz = qlz - sink;
@@ -174,11 +175,11 @@ SHD void icloud_processes_m(const MpConst& K, const MpConstF& F, double& qgz, do
   const float denf = (float)den, denfacf = (float)denfac, dtsf = F.dts;
   const float vtg = (float)vtgz, vtr = (float)vtrz, vts = (float)vtsz;
   double lhi = K.LI00 + K.DC_ICE * tz;
-  double rcpk = cvm / lhi;  // 1 / icpk: every use of icpk here divides by it
+  double rcpk = qdiv(cvm, lhi);  // 1 / icpk: every use of icpk here divides by it
   if (!(p1 >= P_MIN)) return;
   double tc = tz - tice;
   if (tc >= 0.0) {
-    const float dqs0 = (float)(K.ces0 / p1 - qvz);
+    const float dqs0 = (float)(qdiv(K.ces0, p1) - qvz);
     if (qsz > QCMIN) {
       float psacw = 0.0f, psacr = 0.0f, pracs = 0.0f;
       const float qsf = (float)qsz, qlf = (float)qlz, qrf = (float)qrz;
@@ -196,20 +197,20 @@ SHD void icloud_processes_m(const MpConst& K, const MpConstF& F, double& qgz, do
       const float smlt_rate = (F.csmlt[0] * tcf / denf - F.csmlt[1] * dqs0) *
                                   (F.csmlt[2] * sqrtf(qsrho) + F.csmlt[3] * powf(qsrho, 0.65625f) * sqrtf(denfacf)) +
                               F.csmlt[4] * tcf * (psacw + psacr);
-      const double psmlt = fmax(0.0, (double)smlt_rate);
-      const double sink = fmin(qsz, fmin(dts * (psmlt + (double)pracs), tc * rcpk));
+      const double psmlt = qmax(0.0, (double)smlt_rate);
+      const double sink = qmin(qsz, qmin(dts * (psmlt + (double)pracs), tc * rcpk));
       qsz = qsz - sink;
-      const double tmp = fmin(sink, dim(K.qs_mlt, qlz));
+      const double tmp = qmin(sink, dim(K.qs_mlt, qlz));
       qlz = qlz + tmp;
       qrz = qrz + sink - tmp;
       q_liq = q_liq + sink;
       q_sol = q_sol - sink;
       cvm = cvm_of(K, qvz, q_liq, q_sol);
-      tz = tz - sink * lhi / cvm;
+      tz = tz - qdiv(sink * lhi, cvm);
       tc = tz - tice;
     }
     lhi = K.LI00 + K.DC_ICE * tz;
-    rcpk = cvm / lhi;
+    rcpk = qdiv(cvm, lhi);
     if ((qgz > QCMIN) && (tc > 0.0)) {
       float pgacr = 0.0f, pgacw = 0.0f;
       const float qgf = (float)qgz, qrf = (float)qrz, qlf = (float)qlz;
@@ -226,13 +227,13 @@ SHD void icloud_processes_m(const MpConst& K, const MpConstF& F, double& qgz, do
                                   (F.cgmlt[2] * sqrtf(qden) + F.cgmlt[3] * powf(qden, 0.6875f) / powf(denf, 0.25f)) +
                               F.cgmlt[4] * tcf * (pgacw + pgacr);
       double pgmlt = dts * (double)gmlt_rate;
-      pgmlt = fmin(fmax(0.0, pgmlt), fmin(qgz, tc * rcpk));
+      pgmlt = qmin(qmax(0.0, pgmlt), qmin(qgz, tc * rcpk));
       qgz = qgz - pgmlt;
       qrz = qrz + pgmlt;
       q_liq = q_liq + pgmlt;
       q_sol = q_sol - pgmlt;
       cvm = cvm_of(K, qvz, q_liq, q_sol);
-      tz = tz - pgmlt * lhi / cvm;
+      tz = tz - qdiv(pgmlt * lhi, cvm);
     }
   } else {
     if (qiz > 3.0e-7) {
@@ -242,22 +243,22 @@ SHD void icloud_processes_m(const MpConst& K, const MpConstF& F, double& qgz, do
         const float factor = dtsf * denfacf * F.csaci * expf(0.05f * tcf + 0.8125f * logf((float)qsz * denf));
         psaci = factor / (1.0f + factor) * (float)qiz;
       }
-      const double qim = K.qi0_crt / den;
+      const double qim = qdiv(K.qi0_crt, den);
       const double tmp = K.const_vi ? K.fac_i2s : K.fac_i2s * (double)expf(0.025f * tcf);
-      di = fmax(di, QRMIN);
+      di = qmax(di, QRMIN);
       const double q_plus = qiz + di;
       double psaut;
       if (q_plus > (qim + QRMIN)) {
         double dq;
         if (qim > (qiz - di))
-          dq = (0.25 * sq(q_plus - qim)) / di;
+          dq = qdiv(0.25 * sq(q_plus - qim), di);
         else
           dq = qiz - qim;
         psaut = tmp * dq;
       } else {
         psaut = 0.0;
       }
-      const double sink = fmin(0.75 * qiz, (double)psaci + psaut);
+      const double sink = qmin(0.75 * qiz, (double)psaci + psaut);
       qiz = qiz - sink;
       qsz = qsz + sink;
       if (qgz > 1.0e-6) {
@@ -275,7 +276,7 @@ SHD void icloud_processes_m(const MpConst& K, const MpConstF& F, double& qgz, do
         psacr = dtsf * acr3d_f(vts, vtr, qrf, (float)qsz, F.csacr, F.acco[0][1], F.acco[1][1], F.acco[2][1], denf);
       float pgfr = dtsf * F.cgfr[0] / denf * (expf(-F.cgfr[1] * tcf) - 1.0f) * expf(1.75f * logf(qrf * denf));
       const double sink0 = (double)psacr + (double)pgfr;
-      const double factor = fmin(sink0, fmin(qrz, -tc * rcpk)) / fmax(sink0, QRMIN);
+      const double factor = qdiv(qmin(sink0, qmin(qrz, -tc * rcpk)), qmax(sink0, QRMIN));
       const double ps = factor * (double)psacr;
       const double pg = factor * (double)pgfr;
       const double sink = ps + pg;
@@ -285,10 +286,10 @@ SHD void icloud_processes_m(const MpConst& K, const MpConstF& F, double& qgz, do
       q_liq = q_liq - sink;
       q_sol = q_sol + sink;
       cvm = cvm_of(K, qvz, q_liq, q_sol);
-      tz = tz + sink * lhi / cvm;
+      tz = tz + qdiv(sink * lhi, cvm);
     }
     lhi = K.LI00 + K.DC_ICE * tz;
-    rcpk = cvm / lhi;
+    rcpk = qdiv(cvm, lhi);
     if (qsz > 1.0e-7) {
       double sink;
       if (qgz > QRMIN)
@@ -296,12 +297,12 @@ SHD void icloud_processes_m(const MpConst& K, const MpConstF& F, double& qgz, do
                                      F.acco[2][3], denf);
       else
         sink = 0.0;
-      const double qsm = K.qs0_crt / den;
+      const double qsm = qdiv(K.qs0_crt, den);
       if (qsz > qsm) {
         const float factor = dtsf * 1.0e-3f * expf(0.09f * (float)(tz - tice));
         sink = sink + (double)(factor / (1.0f + factor)) * (qsz - qsm);
       }
-      sink = fmin(qsz, sink);
+      sink = qmin(qsz, sink);
       qsz = qsz - sink;
       qgz = qgz + sink;
     }
@@ -315,14 +316,14 @@ SHD void icloud_processes_m(const MpConst& K, const MpConstF& F, double& qgz, do
         pgacw = 0.0;
       }
       if (qrz > 1.0e-6) {
-        pgacr = fmin(dts * (double)acr3d_f(vtg, vtr, (float)qrz, (float)qgz, F.cgacr, F.acco[0][2], F.acco[1][2],
+        pgacr = qmin(dts * (double)acr3d_f(vtg, vtr, (float)qrz, (float)qgz, F.cgacr, F.acco[0][2], F.acco[1][2],
                                            F.acco[2][2], denf),
                      qrz);
       } else {
         pgacr = 0.0;
       }
       double sink = pgacr + pgacw;
-      const double factor = fmin(sink, dim(tice, tz) * rcpk) / fmax(sink, QRMIN);
+      const double factor = qdiv(qmin(sink, dim(tice, tz) * rcpk), qmax(sink, QRMIN));
       pgacr = factor * pgacr;
       pgacw = factor * pgacw;
       sink = pgacr + pgacw;
@@ -332,9 +333,10 @@ SHD void icloud_processes_m(const MpConst& K, const MpConstF& F, double& qgz, do
       q_liq = q_liq - sink;
       q_sol = q_sol + sink;
       cvm = cvm_of(K, qvz, q_liq, q_sol);
-      tz = tz + sink * lhi / cvm;
+      tz = tz + qdiv(sink * lhi, cvm);
     }
   }
 }
 
+}  // namespace SHIELD_ARITH
 }  // namespace shield

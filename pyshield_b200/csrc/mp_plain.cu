@@ -1,5 +1,6 @@
 // Plain FP64 form of the microphysics step. Compiled with -fmad=false so
-// that every multiply and add rounds as the reference's numpy expressions do.
+// that every multiply and add rounds as the reference's numpy expressions do;
+// exp, log, powers and the saturation humidities are those of mp_math.cuh.
 #include "mp_kernel.cuh"
 #include "mp_launch.h"
 
@@ -31,11 +32,6 @@ __global__ void de_ice_kernel(const __grid_constant__ MpArgs A, Fld3 qi_dt, Fld3
 
 namespace {
 
-template <int NW, int G, int MINB, bool FLAGS = false>
-cudaError_t launch_nw(const MpArgs& A, cudaStream_t st) {
-  return launch_step<ColumnLayout<NW, G>, MINB, false, false, FLAGS>(A, st);
-}
-
 __global__ void gather2d(const double* p, int64_t si, int64_t sj, int nx, int64_t n, double* out) {
   for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < n; c += (int64_t)gridDim.x * blockDim.x)
     out[c] = p[(c % nx) * si + (c / nx) * sj];
@@ -45,49 +41,10 @@ __global__ void gather2d(const double* p, int64_t si, int64_t sj, int nx, int64_
 
 int mp_max_levels() { return 256; }
 
-// Launch shape for 81-96 levels: columns per block and the minimum resident
-// blocks per SM given to __launch_bounds__ (which caps the registers per
-// thread). Four columns per block (one 384-thread block per SM) measured
-// fastest: the staging then reads whole 32-byte sectors. 65-80 levels (L79)
-// pack two columns per 5 warps (Packed80).
-#ifndef SHIELD_NW3_G
-#define SHIELD_NW3_G 4
-#endif
-#ifndef SHIELD_NW3_MINB
-#define SHIELD_NW3_MINB 1
-#endif
-// 65..80 levels, plain form: the persistent, input-prefetching kernel (1) or
-// one block per column block (0).
-#ifndef SHIELD_PACK_PERSIST_PLAIN
-#define SHIELD_PACK_PERSIST_PLAIN 0
-#endif
-// 97..128 levels (L127): columns per block of 4 warps each. C96 L127 (ms):
-// 4 columns (512 threads, 128 registers) 6.29, 5 columns (640, 96) 5.94,
-// 6 columns (768, 80) 5.99.
-#ifndef SHIELD_NW4_G
-#define SHIELD_NW4_G 5
-#endif
-
-cudaError_t mp_launch_plain(const MpArgs& A, cudaStream_t st) {
-  const int L = A.nz;
-  if (L <= 32) return launch_nw<1, 4, 2>(A, st);
-  if (L <= 64) return launch_nw<2, 2, 2>(A, st);
-  if (L <= PACK80_LMAX) return launch_step<Packed80, PACK80_MINB, false, SHIELD_PACK_PERSIST_PLAIN>(A, st);
-  if (L <= 96) return launch_nw<3, SHIELD_NW3_G, SHIELD_NW3_MINB>(A, st);
-  if (L <= 128) return launch_nw<4, SHIELD_NW4_G, 1>(A, st);
-  return launch_nw<8, 1, 2>(A, st);
-}
+cudaError_t mp_launch_plain(const MpArgs& A, cudaStream_t st) { return launch_plain_shapes<false>(A, st); }
 
 // The same launches with the column flags recorded (A.flags non-null).
-cudaError_t mp_launch_plain_flags(const MpArgs& A, cudaStream_t st) {
-  const int L = A.nz;
-  if (L <= 32) return launch_nw<1, 4, 2, true>(A, st);
-  if (L <= 64) return launch_nw<2, 2, 2, true>(A, st);
-  if (L <= PACK80_LMAX) return launch_step<Packed80, PACK80_MINB, false, false, true>(A, st);
-  if (L <= 96) return launch_nw<3, SHIELD_NW3_G, SHIELD_NW3_MINB, true>(A, st);
-  if (L <= 128) return launch_nw<4, SHIELD_NW4_G, 1, true>(A, st);
-  return launch_nw<8, 1, 2, true>(A, st);
-}
+cudaError_t mp_launch_plain_flags(const MpArgs& A, cudaStream_t st) { return launch_plain_shapes<true>(A, st); }
 
 cudaError_t mp_launch_mixed(const MpArgs& A, cudaStream_t st);
 

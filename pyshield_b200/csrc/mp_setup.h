@@ -19,24 +19,24 @@ inline void setupm(const ShieldMpConfig& c, MpConst& K) {
   K.GRAV = 9.80665;
   K.RGRAV = 1.0 / K.GRAV;
   K.RDGAS = 287.05;
-  K.RVGAS = 461.50;
-  K.HLV = 2.5e6;
-  K.HLF = 3.3358e5;
-  K.CP_AIR = 1004.6;
+  K.RVGAS = PH_RVGAS;
+  K.HLV = PH_HLV;
+  K.HLF = PH_HLF;
+  K.CP_AIR = PH_CP_AIR;
   K.KAPPA = K.RDGAS / K.CP_AIR;
   K.CP_VAP = 4.0 * K.RVGAS;
   K.CV_AIR = K.CP_AIR - K.RDGAS;
   K.CV_VAP = 3.0 * K.RVGAS;
-  K.C_ICE = 1972.0;
-  K.C_LIQ = 4.1855e3;
-  K.TICE = 273.16;
-  K.E00 = 611.21;
-  K.DC_VAP = K.CP_VAP - K.C_LIQ;
-  K.DC_ICE = K.C_LIQ - K.C_ICE;
-  K.D2ICE = K.DC_VAP + K.DC_ICE;
-  K.LV0 = K.HLV - K.DC_VAP * K.TICE;
-  K.LI00 = K.HLF - K.DC_ICE * K.TICE;
-  K.LI2 = K.LV0 + K.LI00;
+  K.C_ICE = PH_C_ICE;
+  K.C_LIQ = PH_C_LIQ;
+  K.TICE = PH_TICE;
+  K.E00 = PH_E00;
+  K.DC_VAP = PH_DC_VAP;
+  K.DC_ICE = PH_DC_ICE;
+  K.D2ICE = PH_D2ICE;
+  K.LV0 = PH_LV0;
+  K.LI00 = PH_LI00;
+  K.LI2 = PH_LI2;
   K.EPS = K.RDGAS / K.RVGAS;
   K.ZVIR = K.RVGAS / K.RDGAS - 1.0;
   K.T_MIN = 178.0;
@@ -109,6 +109,7 @@ inline void setupm(const ShieldMpConfig& c, MpConst& K) {
   K.iqs_lo_num = K.E00 * std::exp((K.D2ICE * std::log(1.0 - 160.0 / K.TICE) - K.LI2 * 160.0 / (K.T_SAT_MIN * K.TICE)) /
                                   K.RVGAS);
   K.log_10 = std::log(10.0);
+  K.r_log_10 = 1.0 / K.log_10;
   K.tice0 = c.tice - 0.01;
   K.t_wfr = c.tice - 40.0;
   K.c_air = K.CP_AIR;
@@ -199,18 +200,6 @@ inline int set_timestep(const ShieldMpConfig& c, MpConst& K, double timestep, st
 // FP32 copies of the constants used by the mixed form's process rates.
 inline MpConstF to_float(const MpConst& K) {
   MpConstF F;
-  F.qs_e00 = K.E00 / K.RVGAS;
-  F.qw_c1 = K.DC_VAP / K.RVGAS;
-  F.qw_c2 = K.LV0 / K.RVGAS;
-  F.qw_c3 = F.qw_c2 / K.TICE - F.qw_c1 * std::log(K.TICE);
-  F.qi_c1 = K.D2ICE / K.RVGAS;
-  F.qi_c2 = K.LI2 / K.RVGAS;
-  F.qi_c3 = F.qi_c2 / K.TICE - F.qi_c1 * std::log(K.TICE);
-  F.qs_t0 = K.TICE;
-  F.qs_tmin = K.T_SAT_MIN;
-  F.qs_thi = K.TICE + 102.0;
-  F.qi_lo = K.iqs_lo_num / (K.RVGAS * K.T_SAT_MIN);
-  F.qi_lo_dq = (K.D2ICE + K.LI2 / K.T_SAT_MIN) / (K.RVGAS * K.T_SAT_MIN);
   F.qs_rtw = 1.0 / (K.tice - K.t_wfr);
   F.E00 = (float)K.E00;
   F.DC_VAP = (float)K.DC_VAP;

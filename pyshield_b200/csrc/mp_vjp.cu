@@ -26,6 +26,11 @@
 //     the CCN sums, then a point launch that writes the gradients.
 // Branches follow the forward at the given input (the VJP of the piecewise
 // smooth map on the branch it takes).
+//
+// The replay and the reverses keep the reference's rounding (mp_ieee.cu
+// says why the differentiated forward does): over a window, vapour settles
+// on saturation to the last place, and the sign of qv - qs decides branches.
+#define SHIELD_IEEE
 #include <cuda_runtime.h>
 
 #include "mp_adjoint.cuh"
@@ -237,16 +242,16 @@ SHD void w_update_b(int k, double w, double dm, double flux, double vt, double f
   const double wo_b = w_b;
   if (k == 0) {
     const double Dd = dm - flux;
-    const double wo = (dm * w + flux * vt) / Dd;
-    const double N_b = wo_b / Dd, Dd_b = -wo_b * wo / Dd;
+    const double wo = qdiv(dm * w + flux * vt, Dd);
+    const double N_b = qdiv(wo_b, Dd), Dd_b = qdiv(-wo_b * wo, Dd);
     w_b = N_b * dm;
     dm_b += N_b * w + Dd_b;
     flux_b += N_b * vt - Dd_b;
     vt_b += N_b * flux;
   } else {
     const double Dd = dm + fp - flux;
-    const double wo = (dm * w - fp * vp + flux * vt) / Dd;
-    const double N_b = wo_b / Dd, Dd_b = -wo_b * wo / Dd;
+    const double wo = qdiv(dm * w - fp * vp + flux * vt, Dd);
+    const double N_b = qdiv(wo_b, Dd), Dd_b = qdiv(-wo_b * wo, Dd);
     w_b = N_b * dm;
     dm_b += N_b * w + Dd_b;
     fp_b += -N_b * vp + Dd_b;
@@ -267,11 +272,11 @@ SHD void mono_slope_coeffs(double qp, double q, double qn, int k, int L, double 
   const double dqn = 0.5 * (qn - q);
   const double s = dq + dqn;
   const double A1 = fabs(s), A2 = 0.5 * q;
-  const double v0 = 0.5 * fmin(A1, A2);
+  const double v0 = 0.5 * qmin(A1, A2);
   double v0_b = 0.0, dq_b = 0.0, dqn_b = 0.0;
   if (dq * dqn <= 0.0) {
     if (dq > 0.0) {
-      const double m2 = fmin(dq, -dqn);
+      const double m2 = qmin(dq, -dqn);
       if (min_first(v0, m2))
         v0_b = v_b;
       else if (min_first(dq, -dqn))
@@ -327,14 +332,14 @@ SHD FallRec implicit_fall_rec(Column<NW>& C, double q, double vt, double dz, dou
   const double qmass = valid ? q * dp1 : 0.0;
   const double ddp = C.prev(R.dd);
   R.D = dz + R.dd;
-  R.a = qmass / R.D;
-  R.b = (C.k == 0) ? 0.0 : ddp / R.D;
+  R.a = qdiv(qmass, R.D);
+  R.b = (C.k == 0) ? 0.0 : qdiv(ddp, R.D);
   if (!valid) {
     R.a = 0.0;
     R.b = 0.0;
   }
   R.r = C.scan_affine(R.a, R.b);
-  R.q1 = valid ? R.r * dz / dp1 : q;
+  R.q1 = valid ? qdiv(R.r * dz, dp1) : q;
   R.flux = valid ? R.dd * R.r : 0.0;
   return R;
 }
@@ -345,9 +350,9 @@ SHD void implicit_fall_b(Column<NW>& C, const FallRec& R, double q, double dz, d
   const int k = C.k, L = C.L;
   double r_b = 0.0, dd_b = 0.0;
   if (valid) {
-    r_b = q_b * dz / dp1 + flux_b * R.dd;
-    dz_b += q_b * R.r / dp1;
-    dp1_b -= q_b * R.q1 / dp1;
+    r_b = qdiv(q_b * dz, dp1) + flux_b * R.dd;
+    dz_b += qdiv(q_b * R.r, dp1);
+    dp1_b -= qdiv(q_b * R.q1, dp1);
     dd_b = flux_b * R.r;
   }
   double bv[1] = {R.b}, bn[1];
@@ -359,9 +364,9 @@ SHD void implicit_fall_b(Column<NW>& C, const FallRec& R, double q, double dz, d
   if (valid) {
     const double a_b = lam;
     const double b_b = (k > 0) ? lam * rp : 0.0;
-    const double qmass_b = a_b / R.D;
-    const double D_b = -a_b * R.a / R.D - b_b * R.b / R.D;
-    ddp_b = b_b / R.D;
+    const double qmass_b = qdiv(a_b, R.D);
+    const double D_b = qdiv(-a_b * R.a, R.D) - qdiv(b_b * R.b, R.D);
+    ddp_b = qdiv(b_b, R.D);
     dz_b += D_b;
     dd_b += D_b;
     q_b = qmass_b * dp1;
@@ -398,12 +403,12 @@ SHD void sedi_heat_b(Column<NW>& C, const MpConst& K, double tz, double dz1, dou
   double a, b, D = 1.0, tmp = 1.0;
   if (k == 0) {
     tmp = cvn + flux * c_cond;
-    a = tz + flux * dgz / tmp;
+    a = tz + qdiv(flux * dgz, tmp);
     b = 0.0;
   } else {
     D = cvn + c_cond * flux;
-    a = ((cvn + c_cond * (flux - fp)) * tz + dgz * (fp + flux)) / D;
-    b = fp * c_cond / D;
+    a = qdiv((cvn + c_cond * (flux - fp)) * tz + dgz * (fp + flux), D);
+    b = qdiv(fp * c_cond, D);
   }
   if (!valid) {
     a = tz;
@@ -420,19 +425,19 @@ SHD void sedi_heat_b(Column<NW>& C, const MpConst& K, double tz, double dz1, dou
   double cvn_b = 0.0, dgz_b = 0.0;
   if (k == 0) {
     const double u = flux * dgz;
-    const double u_b = lam / tmp, tmp_b = -lam * u / (tmp * tmp);
+    const double u_b = qdiv(lam, tmp), tmp_b = qdiv(-lam * u, tmp * tmp);
     Sb.tz = lam;
     flux_b += u_b * dgz + tmp_b * c_cond;
     dgz_b += u_b * flux;
     cvn_b += tmp_b;
   } else {
     const double b_b = lam * xp;
-    const double N_b = lam / D;
-    const double D_b = -lam * a / D - b_b * b / D;
+    const double N_b = qdiv(lam, D);
+    const double D_b = qdiv(-lam * a, D) - qdiv(b_b * b, D);
     Sb.tz = N_b * (cvn + c_cond * (flux - fp));
     cvn_b += N_b * tz + D_b;
     flux_b += N_b * (c_cond * tz + dgz) + D_b * c_cond;
-    fp_b += N_b * (dgz - c_cond * tz) + b_b * c_cond / D;
+    fp_b += N_b * (dgz - c_cond * tz) + qdiv(b_b * c_cond, D);
     dgz_b += N_b * (fp + flux);
   }
   dz1_b += -0.5 * K.GRAV * dgz_b;
@@ -477,8 +482,8 @@ SHD void sedimentation_b(Column<NW>& C, const MpConst& K, bool valid, const LevS
     for (int n = 0; n < 3; ++n) {
       const double qmass = valid ? qq[n] * dp1 : 0.0;
       D[n] = dz + dd[n];
-      ra[n] = qmass / D[n];
-      rb[n] = (k == 0) ? 0.0 : ddp[n] / D[n];
+      ra[n] = qdiv(qmass, D[n]);
+      rb[n] = (k == 0) ? 0.0 : qdiv(ddp[n], D[n]);
       if (!valid) {
         ra[n] = 0.0;
         rb[n] = 0.0;
@@ -489,11 +494,11 @@ SHD void sedimentation_b(Column<NW>& C, const MpConst& K, bool valid, const LevS
 #pragma unroll
     for (int n = 0; n < 3; ++n) flux[n] = valid ? dd[n] * r[n] : 0.0;
     const double dm_i = dp1 * (1.0 + S1.qv + S1.ql + S1.qr + S1.qi + S1.qs + S1.qg);
-    const double qi2 = (fi && valid) ? r[0] * dz / dp1 : S1.qi;
+    const double qi2 = (fi && valid) ? qdiv(r[0] * dz, dp1) : S1.qi;
     const double dm_s = dp1 * (1.0 + S1.qv + S1.ql + S1.qr + qi2 + S1.qs + S1.qg);
-    const double qs2 = (fs && valid) ? r[1] * dz / dp1 : S1.qs;
+    const double qs2 = (fs && valid) ? qdiv(r[1] * dz, dp1) : S1.qs;
     const double dm_g = dp1 * (1.0 + S1.qv + S1.ql + S1.qr + qi2 + qs2 + S1.qg);
-    const double qg2 = (fg && valid) ? r[2] * dz / dp1 : S1.qg;
+    const double qg2 = (fg && valid) ? qdiv(r[2] * dz, dp1) : S1.qg;
     const double nv[6] = {flux[0], vti, flux[1], vts, flux[2], vtg};
     double pv[6];
     C.template prevN<6>(nv, pv);
@@ -567,9 +572,9 @@ SHD void sedimentation_b(Column<NW>& C, const MpConst& K, bool valid, const LevS
     double r_b[3] = {0.0, 0.0, 0.0};
     if (valid) {
       if (fg) {
-        r_b[2] += Sb.qg * dz / dp1;
-        Ab.dz += Sb.qg * r[2] / dp1;
-        Ab.dp1 -= Sb.qg * qg2 / dp1;
+        r_b[2] += qdiv(Sb.qg * dz, dp1);
+        Ab.dz += qdiv(Sb.qg * r[2], dp1);
+        Ab.dp1 -= qdiv(Sb.qg * qg2, dp1);
         Sb.qg = 0.0;
       }
       {
@@ -578,9 +583,9 @@ SHD void sedimentation_b(Column<NW>& C, const MpConst& K, bool valid, const LevS
         Sb.qv += t, Sb.ql += t, Sb.qr += t, Sb.qi += t, Sb.qs += t, Sb.qg += t;
       }
       if (fs) {
-        r_b[1] += Sb.qs * dz / dp1;
-        Ab.dz += Sb.qs * r[1] / dp1;
-        Ab.dp1 -= Sb.qs * qs2 / dp1;
+        r_b[1] += qdiv(Sb.qs * dz, dp1);
+        Ab.dz += qdiv(Sb.qs * r[1], dp1);
+        Ab.dp1 -= qdiv(Sb.qs * qs2, dp1);
         Sb.qs = 0.0;
       }
       {
@@ -589,9 +594,9 @@ SHD void sedimentation_b(Column<NW>& C, const MpConst& K, bool valid, const LevS
         Sb.qv += t, Sb.ql += t, Sb.qr += t, Sb.qi += t, Sb.qs += t, Sb.qg += t;
       }
       if (fi) {
-        r_b[0] += Sb.qi * dz / dp1;
-        Ab.dz += Sb.qi * r[0] / dp1;
-        Ab.dp1 -= Sb.qi * qi2 / dp1;
+        r_b[0] += qdiv(Sb.qi * dz, dp1);
+        Ab.dz += qdiv(Sb.qi * r[0], dp1);
+        Ab.dp1 -= qdiv(Sb.qi * qi2, dp1);
         Sb.qi = 0.0;
       }
       {
@@ -625,9 +630,9 @@ SHD void sedimentation_b(Column<NW>& C, const MpConst& K, bool valid, const LevS
       for (int n = 0; n < 3; ++n) {
         const double a_b = lam[n];
         const double b_b = (k > 0) ? lam[n] * rp[n] : 0.0;
-        const double qmass_b = a_b / D[n];
-        const double D_b = -a_b * ra[n] / D[n] - b_b * rb[n] / D[n];
-        ddp_b[n] = b_b / D[n];
+        const double qmass_b = qdiv(a_b, D[n]);
+        const double D_b = qdiv(-a_b * ra[n], D[n]) - qdiv(b_b * rb[n], D[n]);
+        ddp_b[n] = qdiv(b_b, D[n]);
         Ab.dz += D_b;
         dd_b[n] += D_b;
         q_b[n] = qmass_b * dp1;
@@ -768,7 +773,7 @@ SHD void ws_scatter(double* const (&dst)[NF], const double* tiles, int64_t ncol,
 // when qi becomes qi0_max.
 SHD int de_ice_point(const MpConst& K, double& qi, double& qs, double qi_dt) {
   const double qio = qi - K.timestep * qi_dt;
-  const double qin = fmax(qio, K.qi0_max);
+  const double qin = qmax(qio, K.qi0_max);
   if (!(qi > qin)) return 0;
   qs = qs + qi - qin;
   qi = qin;
@@ -1029,7 +1034,7 @@ __global__ void __launch_bounds__(PT_THREADS, SHIELD_VJP_PT_MINB) vjp_update_pt(
   const double cq[6] = {cot(OUT_QV_DT), cot(OUT_QL_DT), cot(OUT_QR_DT), cot(OUT_QI_DT), cot(OUT_QS_DT), cot(OUT_QG_DT)};
   const double qf[6] = {S.qv, S.ql, S.qr, S.qi, S.qs, S.qg};
   const double dp0 = delp;
-  const double omq0 = dp0 / dp1, omq = dp1 / dp0;
+  const double omq0 = qdiv(dp0, dp1), omq = qdiv(dp1, dp0);
   double qfb[6], qin_b[6], omq_b = 0.0, omq0_b = 0.0;
 #pragma unroll
   for (int n = 0; n < 6; ++n) {
@@ -1041,7 +1046,7 @@ __global__ void __launch_bounds__(PT_THREADS, SHIELD_VJP_PT_MINB) vjp_update_pt(
     omq0_b += q0_b * qin[n];
   }
   const double cvm = K.c_air + S.qv * K.c_vap + (S.qr + S.ql) * K.C_LIQ + (S.qi + S.qs + S.qg) * K.C_ICE;
-  const double gpt = cot(OUT_PT_DT) * rdt / K.CP_AIR;
+  const double gpt = qdiv(cot(OUT_PT_DT) * rdt, K.CP_AIR);
   LevState Sb;
   Sb.tz = gpt * cvm;
   const double pt_b = -gpt * cvm;
@@ -1058,16 +1063,16 @@ __global__ void __launch_bounds__(PT_THREADS, SHIELD_VJP_PT_MINB) vjp_update_pt(
   // qa_dt = rdt (qaz_out / ntimes - qa0) (without do_qa, which leaves both)
   double qa_b = cot(OUT_QAZ), qa0_b = 0.0;
   if (!K.do_qa) {
-    qa_b += cot(OUT_QA_DT) * rdt / (double)K.ntimes;
+    qa_b += qdiv(cot(OUT_QA_DT) * rdt, (double)K.ntimes);
     qa0_b = -cot(OUT_QA_DT) * rdt;
   }
   store_lev(W.as(AS_QV) + p, np, Sb);
-  W.as(AS_DP1)[p] = omq_b / dp0 - omq0_b * omq0 / dp1;
+  W.as(AS_DP1)[p] = qdiv(omq_b, dp0) - qdiv(omq0_b * omq0, dp1);
   W.as(AS_P1)[p] = 0.0;
   W.as(AS_CCN)[p] = 0.0;
   W.as(AS_CPRAUT)[p] = 0.0;
   W.as(AS_PT)[p] = pt_b;
-  W.as(AS_DELP)[p] = -omq_b * omq / dp0 + omq0_b / dp1;
+  W.as(AS_DELP)[p] = qdiv(-omq_b * omq, dp0) + qdiv(omq0_b, dp1);
   W.as(AS_DZ0)[p] = 0.0;
 #pragma unroll
   for (int n = 0; n < 6; ++n) W.as(AS_QIN0 + n)[p] = qin_b[n];
@@ -1122,9 +1127,9 @@ __global__ void __launch_bounds__(32 * NW * G, MINB) vjp_momentum_kernel(const _
       b = 0.0;
     } else {
       D = delp + mp;
-      au = delp * u0 / D;
-      av = delp * v0 / D;
-      b = mp / D;
+      au = qdiv(delp * u0, D);
+      av = qdiv(delp * v0, D);
+      b = qdiv(mp, D);
     }
     double u1, v1;
     C.scan_affine2(au, b, av, b, u1, v1);
@@ -1147,12 +1152,12 @@ __global__ void __launch_bounds__(32 * NW * G, MINB) vjp_momentum_kernel(const _
         v0_b += lam[1];
       } else {
         const double b_b = lam[0] * pp[0] + lam[1] * pp[1];
-        u0_b += lam[0] * delp / D;
-        v0_b += lam[1] * delp / D;
-        delp_b += lam[0] * u0 / D + lam[1] * v0 / D;
-        const double D_b = -lam[0] * au / D - lam[1] * av / D - b_b * b / D;
+        u0_b += qdiv(lam[0] * delp, D);
+        v0_b += qdiv(lam[1] * delp, D);
+        delp_b += qdiv(lam[0] * u0, D) + qdiv(lam[1] * v0, D);
+        const double D_b = qdiv(-lam[0] * au, D) - qdiv(lam[1] * av, D) - qdiv(b_b * b, D);
         delp_b += D_b;
-        mp_b = b_b / D + D_b;
+        mp_b = qdiv(b_b, D) + D_b;
       }
     }
     double mv[1] = {mp_b}, mn[1];
@@ -1216,11 +1221,11 @@ __global__ void __launch_bounds__(PT_THREADS, SHIELD_VJP_PT_MINB) vjp_icloud_pt(
   double q_liq, q_sol, cvm;
   icloud_melt_freeze(K, S1.qv, S1.ql, S1.qr, S1.qi, S1.qs, S1.qg, S1.tz, den, q_liq, q_sol, cvm);
   const double hq = h_var * S1.qi;
-  const double inner = fmax(QVMIN, hq);
+  const double inner = qmax(QVMIN, hq);
   double sl = 0.0, di = inner;
   if (K.z_slope_ice) {
     sl = W.ss(it, SS_SL_I)[p];
-    di = fmax(sl, inner);
+    di = qmax(sl, inner);
   }
   const IcState Z0{S1.qg, S1.qi, S1.ql, S1.qr, S1.qs, S1.tz, q_liq, q_sol, cvm};
   const IcIn I{S1.qv, den, denfac, vtg, vtr, vts, p1, di};
@@ -1280,11 +1285,11 @@ __global__ void __launch_bounds__(PT_THREADS, SHIELD_VJP_PT_MINB) vjp_autoconv_p
     autoconv_no_subgrid_var_b(K, W3.ql, W3.qr, W3.tz, den, ccn, c_praut, Sb.ql, Sb.qr, den_b, ccn_b, cpr_b);
   } else {
     const double hq = h_var * W3.ql;
-    const double inner = fmax(QVMIN, hq);
+    const double inner = qmax(QVMIN, hq);
     double sl = 0.0, dl = inner;
     if (K.z_slope_liq) {
       sl = W.ss(it, PASS ? SS_SL_B : SS_SL_A)[p];
-      dl = fmax(sl, inner);
+      dl = qmax(sl, inner);
     }
     double dl_b = 0.0;
     autoconv_subgrid_var_b(K, W3.ql, W3.qr, W3.tz, den, ccn, c_praut, dl, Sb.ql, Sb.qr, den_b, ccn_b, cpr_b, dl_b);
@@ -1355,17 +1360,17 @@ __global__ void __launch_bounds__(PT_THREADS, SHIELD_VJP_PT_MINB) vjp_revap1_pt(
     const double dz0 = fz.p[i * fz.si + j * fz.sj + (int64_t)q.k * fz.sk];
     const double dp1 = W.sp(SP_DP1)[p], dz1 = W.ss(it, SS_DZ1)[p], tz0 = W.ckf(it, CKF_E0 + 6)[p];
     const double aden = W.as(AS_DEN)[p] + den_b, adenfac = W.as(AS_DENFAC)[p] + denfac_b;
-    const double den0 = -dp1 / (K.GRAV * dz0);
-    const double dn_b = aden - adenfac * 0.5 * denfac / den;
+    const double den0 = qdiv(-dp1, K.GRAV * dz0);
+    const double dn_b = aden - qdiv(adenfac * 0.5 * denfac, den);
     double dz1_b = -W.as(AS_DZ)[p];
-    const double den0_b = dn_b * dz0 / dz1;
-    double dz0_b = dn_b * den0 / dz1;
-    dz1_b -= dn_b * den / dz1;
-    dz0_b += dz1_b * tz0 / pt;
-    Sb.tz += dz1_b * dz0 / pt;
-    const double pt_b = -dz1_b * dz1 / pt;
-    const double dp1_b = -den0_b / (K.GRAV * dz0);
-    dz0_b += den0_b * dp1 / (K.GRAV * dz0 * dz0);
+    const double den0_b = qdiv(dn_b * dz0, dz1);
+    double dz0_b = qdiv(dn_b * den0, dz1);
+    dz1_b -= qdiv(dn_b * den, dz1);
+    dz0_b += qdiv(dz1_b * tz0, pt);
+    Sb.tz += qdiv(dz1_b * dz0, pt);
+    const double pt_b = qdiv(-dz1_b * dz1, pt);
+    const double dp1_b = qdiv(-den0_b, K.GRAV * dz0);
+    dz0_b += qdiv(den0_b * dp1, K.GRAV * dz0 * dz0);
     W.as(AS_DZ0)[p] += dz0_b;
     W.as(AS_PT)[p] += pt_b;
     W.as(AS_DP1)[p] += dp1_b;
@@ -1607,9 +1612,9 @@ __global__ void __launch_bounds__(32 * NW * G, MINB) vjp_fixneg_kernel(const __g
     // c_praut = cpaut (ccn RHOR)^(-1/3); ccn is one value per column
     double ccn_b = C.colsum(valid ? T(XT_CCN) : 0.0);
     const double cpr_b = C.colsum(valid ? T(XT_CPR) : 0.0);
-    if (!K.prog_ccn) ccn_b += cpr_b * W.sc(SC_CPRAUT)[col] * (-1.0 / 3.0) / W.sc(SC_CCN)[col];
+    if (!K.prog_ccn) ccn_b += qdiv(cpr_b * W.sc(SC_CPRAUT)[col] * (-1.0 / 3.0), W.sc(SC_CCN)[col]);
     if (k == 0) W.sc(SC_CCNB)[col] = ccn_b;
-    const double omq = delp / P.dp1;
+    const double omq = qdiv(delp, P.dp1);
     const LevState S0{qin[0] * omq, qin[1] * omq, qin[2] * omq, qin[3] * omq, qin[4] * omq, qin[5] * omq, pt, 0.0};
     if (K.fix_negative) {
       LevState S1 = S0;
@@ -1629,7 +1634,7 @@ __global__ void __launch_bounds__(32 * NW * G, MINB) vjp_fixneg_kernel(const __g
         if (k == 0) {
           for (int kk = 1; kk < L; ++kk) {
             const double pq = wq[kk - 1];
-            if (pq < 0.0) wq[kk] = wq[kk] + pq * wd[kk - 1] / wd[kk];
+            if (pq < 0.0) wq[kk] = wq[kk] + qdiv(pq * wd[kk - 1], wd[kk]);
           }
         }
         C.sync();
@@ -1641,15 +1646,15 @@ __global__ void __launch_bounds__(32 * NW * G, MINB) vjp_fixneg_kernel(const __g
       C.bcast2(qv3, P.dp1, L - 1, qb, db);
       C.bcast2(qv3, P.dp1, L - 2, qb1, db1);
       if ((qb < 0.0) && (qb1 > 0.0)) {
-        const double dq = fmin(-qb * db, qb1 * db1);
+        const double dq = qmin(-qb * db, qb1 * db1);
         double c = 0.0;
         if (k == L - 2) {
-          c = -Sb.qv / P.dp1;
-          Ab.dp1 += Sb.qv * dq / (P.dp1 * P.dp1);
+          c = qdiv(-Sb.qv, P.dp1);
+          Ab.dp1 += qdiv(Sb.qv * dq, P.dp1 * P.dp1);
         }
         if (k == L - 1) {
-          c = Sb.qv / P.dp1;
-          Ab.dp1 -= Sb.qv * dq / (P.dp1 * P.dp1);
+          c = qdiv(Sb.qv, P.dp1);
+          Ab.dp1 -= qdiv(Sb.qv * dq, P.dp1 * P.dp1);
         }
         const double dq_b = C.colsum(c);
         if (min_first(-qb * db, qb1 * db1)) {
@@ -1676,9 +1681,9 @@ __global__ void __launch_bounds__(32 * NW * G, MINB) vjp_fixneg_kernel(const __g
             const double pq = wq[kk - 1];
             if (pq < 0.0) {
               const double gq = wqb[kk];
-              wqb[kk - 1] += gq * wd[kk - 1] / wd[kk];
-              wdb[kk - 1] += gq * pq / wd[kk];
-              wdb[kk] -= gq * pq * wd[kk - 1] / (wd[kk] * wd[kk]);
+              wqb[kk - 1] += qdiv(gq * wd[kk - 1], wd[kk]);
+              wdb[kk - 1] += qdiv(gq * pq, wd[kk]);
+              wdb[kk] -= qdiv(gq * pq * wd[kk - 1], wd[kk] * wd[kk]);
             }
           }
         }
@@ -1726,22 +1731,22 @@ __global__ void __launch_bounds__(PT_THREADS, SHIELD_VJP_PT_MINB) vjp_init_pt(co
   double qin_b[6];
 #pragma unroll
   for (int n = 0; n < 6; ++n) qin_b[n] = W.as(AS_QIN0 + n)[p];
-  const double omq = delp / dp1;
+  const double omq = qdiv(delp, dp1);
   if (K.fix_negative)
     fix_negative_point_b(K, qin[0] * omq, qin[1] * omq, qin[2] * omq, qin[3] * omq, qin[4] * omq, qin[5] * omq, pt,
                          Sb.qv, Sb.ql, Sb.qr, Sb.qi, Sb.qs, Sb.qg, Sb.tz);
   if (!K.prog_ccn && K.use_ccn && k == L - 1) {
     // ccn = ccn0 RDGAS tz / p1 of the bottom level, tz = pt there
     const double ccn_b = W.sc(SC_CCNB)[col], ccn = W.sc(SC_CCN)[col];
-    pt_b += ccn_b * ccn / pt;
-    Ab_p1 -= ccn_b * ccn / W.sp(SP_P1)[p];
+    pt_b += qdiv(ccn_b * ccn, pt);
+    Ab_p1 -= qdiv(ccn_b * ccn, W.sp(SP_P1)[p]);
   }
   // p1 = den0 RDGAS pt, den0 = -dp1 / (g dz0)
-  const double den0 = -dp1 / (K.GRAV * dz0);
+  const double den0 = qdiv(-dp1, K.GRAV * dz0);
   const double den0_b = Ab_p1 * K.RDGAS * pt;
   pt_b += Ab_p1 * den0 * K.RDGAS;
-  Ab_dp1 -= den0_b / (K.GRAV * dz0);
-  dz0_b += den0_b * dp1 / (K.GRAV * dz0 * dz0);
+  Ab_dp1 -= qdiv(den0_b, K.GRAV * dz0);
+  dz0_b += qdiv(den0_b * dp1, K.GRAV * dz0 * dz0);
   // q = q_in omq, omq = delp / dp1, dp1 = delp (1 - qv_in)
   const double sq_b[6] = {Sb.qv, Sb.ql, Sb.qr, Sb.qi, Sb.qs, Sb.qg};
   double omq_b = 0.0;
@@ -1750,8 +1755,8 @@ __global__ void __launch_bounds__(PT_THREADS, SHIELD_VJP_PT_MINB) vjp_init_pt(co
     omq_b += sq_b[n] * qin[n];
     qin_b[n] += sq_b[n] * omq;
   }
-  delp_b += omq_b / dp1;
-  Ab_dp1 -= omq_b * omq / dp1;
+  delp_b += qdiv(omq_b, dp1);
+  Ab_dp1 -= qdiv(omq_b * omq, dp1);
   delp_b += Ab_dp1 * (1.0 - qin[0]);
   qin_b[0] -= Ab_dp1 * delp;
   pt_b += Sb.tz;
