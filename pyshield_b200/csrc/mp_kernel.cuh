@@ -105,16 +105,113 @@ struct Column {
   // column here (control flow around vertical operations must be uniform
   // over the barrier's threads)
   SHD bool group_any(bool p) { return any(p); }
-  // any() with the group's any() from the same exchange (one column here)
-  SHD bool any_group(bool p, bool& g) {
-    g = any(p);
-    return g;
+  // the column's any(p), the barrier group's, and x at level k - 1, from one
+  // exchange
+  SHD void any_prev(bool p, double x, bool& r, bool& g, double& px) {
+    const bool m = __any_sync(FULLMASK, p);
+    px = __shfl_up_sync(FULLMASK, x, 1);
+    r = m;
+    if (NW > 1) {
+      double* s = slot();
+      unsigned* su = reinterpret_cast<unsigned*>(s + NW);
+      if (lane == 31) {
+        s[w] = x;
+        su[w] = m ? 1u : 0u;
+      }
+      sync();
+      if (lane == 0 && w > 0) px = s[w - 1];
+      unsigned o = 0;
+#pragma unroll
+      for (int u = 0; u < NW; ++u) o |= su[u];
+      r = o != 0;
+    }
+    g = r;
   }
-  SHD void any3_group(bool a, bool b, bool c, bool& ra, bool& rb, bool& rc, bool& ga, bool& gb, bool& gc) {
-    any3(a, b, c, ra, rb, rc);
-    ga = ra;
-    gb = rb;
-    gc = rc;
+  // the first level where p holds (1 << 30: none) and x at level k - 1, from
+  // one exchange
+  template <int N>
+  SHD int first_prevN(bool p, const double (&x)[N], double (&px)[N]) {
+    const unsigned m = __ballot_sync(FULLMASK, p);
+    const int mine = m ? 32 * w + __ffs(m) - 1 : 1 << 30;
+#pragma unroll
+    for (int n = 0; n < N; ++n) px[n] = __shfl_up_sync(FULLMASK, x[n], 1);
+    if (NW == 1) return mine;
+    double* s = slot();
+    int* si = reinterpret_cast<int*>(s + N * NW);
+    if (lane == 31) {
+#pragma unroll
+      for (int n = 0; n < N; ++n) s[N * w + n] = x[n];
+      si[w] = mine;
+    }
+    sync();
+    if (lane == 0 && w > 0) {
+#pragma unroll
+      for (int n = 0; n < N; ++n) px[n] = s[N * (w - 1) + n];
+    }
+    int f = si[0];
+#pragma unroll
+    for (int u = 1; u < NW; ++u) f = min(f, si[u]);
+    return f;
+  }
+  // N top-down affine scans (scanN), their values at level k - 1, and the
+  // column's any() of N flags, from one exchange
+  template <int N>
+  SHD void scanN_prev_any(const double (&a)[N], const double (&b)[N], bool (&p)[N], double (&x)[N], double (&xp)[N]) {
+    double A[N], B[N];
+    unsigned m = 0;
+#pragma unroll
+    for (int n = 0; n < N; ++n) {
+      A[n] = a[n];
+      B[n] = b[n];
+      m |= (__any_sync(FULLMASK, p[n]) ? 1u : 0u) << n;
+    }
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+#pragma unroll
+      for (int n = 0; n < N; ++n) {
+        const double pA = __shfl_up_sync(FULLMASK, A[n], d);
+        const double pB = __shfl_up_sync(FULLMASK, B[n], d);
+        if (lane >= d) {
+          A[n] = A[n] + B[n] * pA;
+          B[n] = B[n] * pB;
+        }
+      }
+    }
+    if (NW > 1) {
+      double* s = slot();
+      unsigned* su = reinterpret_cast<unsigned*>(s + 2 * N * NW);
+      if (lane == 31) {
+#pragma unroll
+        for (int n = 0; n < N; ++n) {
+          s[2 * N * w + 2 * n] = A[n];
+          s[2 * N * w + 2 * n + 1] = B[n];
+        }
+        su[w] = m;
+      }
+      sync();
+#pragma unroll
+      for (int n = 0; n < N; ++n) {
+        double X = 0.0;
+        for (int u = 0; u < w; ++u) X = s[2 * N * u + 2 * n] + s[2 * N * u + 2 * n + 1] * X;
+        x[n] = A[n] + B[n] * X;
+        xp[n] = X;
+      }
+      m = su[0];
+#pragma unroll
+      for (int u = 1; u < NW; ++u) m |= su[u];
+    } else {
+#pragma unroll
+      for (int n = 0; n < N; ++n) {
+        x[n] = A[n];
+        xp[n] = 0.0;
+      }
+    }
+#pragma unroll
+    for (int n = 0; n < N; ++n) {
+      const double v = __shfl_up_sync(FULLMASK, x[n], 1);
+      if (lane > 0) xp[n] = v;
+      p[n] = (m >> n) & 1u;
+    }
   }
   SHD int min_int(int v) {
     v = __reduce_min_sync(FULLMASK, v);
@@ -223,17 +320,27 @@ struct Column {
       for (int n = 0; n < N; ++n) px[n] = s[N * (w - 1) + n];
     }
   }
-  // values at levels k - 1 and k + 1 with one barrier
-  SHD void nbrs(double x, double& xp, double& xn) {
-    xp = __shfl_up_sync(FULLMASK, x, 1);
-    xn = __shfl_down_sync(FULLMASK, x, 1);
+  // values at levels k - 1 and k + 1 of N fields with one barrier
+  template <int N>
+  SHD void nbrsN(const double (&x)[N], double (&xp)[N], double (&xn)[N]) {
+#pragma unroll
+    for (int n = 0; n < N; ++n) {
+      xp[n] = __shfl_up_sync(FULLMASK, x[n], 1);
+      xn[n] = __shfl_down_sync(FULLMASK, x[n], 1);
+    }
     if (NW == 1) return;
     double* s = slot();
-    if (lane == 0) s[2 * w] = x;
-    if (lane == 31) s[2 * w + 1] = x;
+#pragma unroll
+    for (int n = 0; n < N; ++n) {
+      if (lane == 0) s[2 * (N * w + n)] = x[n];
+      if (lane == 31) s[2 * (N * w + n) + 1] = x[n];
+    }
     sync();
-    if (lane == 0 && w > 0) xp = s[2 * w - 1];
-    if (lane == 31 && w < NW - 1) xn = s[2 * w + 2];
+#pragma unroll
+    for (int n = 0; n < N; ++n) {
+      if (lane == 0 && w > 0) xp[n] = s[2 * (N * (w - 1) + n) + 1];
+      if (lane == 31 && w < NW - 1) xn[n] = s[2 * (N * (w + 1) + n)];
+    }
   }
   // three column any() flags with one barrier
   SHD void any3(bool a, bool b, bool c, bool& ra, bool& rb, bool& rc) {
@@ -460,21 +567,24 @@ struct Column {
 // Every vertical operation is segmented by column: a value never enters
 // arithmetic with another column's (the warp scans combine lanes of one
 // column only, the carries between warps come from that column's warps, the
-// any/min reductions and broadcasts keep a slot per column). A column spans
-// whole warps except at its ends, so a warp holds parts of at most two
-// segments (L > 32): the one holding its lane 0 (head) and the one holding
-// its lane 31 (tail). Control flow around a vertical operation must be
-// uniform over the whole group (group_any), not only over a column.
+// any/first reductions and broadcasts keep a slot per column). A column
+// spans SPAN = 3 warps, whole ones except at its ends, so a warp holds parts
+// of at most two segments: the one holding its lane 0 (head) and the one
+// holding its lane 31 (tail). Control flow around a vertical operation must
+// be uniform over the whole group (the group's any()), not only over a
+// column. The idle tail reads the last column's slots; its values reach
+// nothing.
 template <int NWG, int P>
 struct PackedColumn {
   static constexpr int T = 32 * NWG;   // threads of the group
   static constexpr int LMAX = T / P;   // longest column that fits
   static constexpr int WP = LMAX + 1;  // pitch of the work rows
   static constexpr int SCR = 8 * NWG + 8 + 4 * (P + 1);  // scratch doubles per parity
-  // t: thread of the group; c: its column slot (P for the idle tail); k:
-  // its level. The segment's extent is derived from these when needed,
-  // which keeps the per-thread state small.
+  static constexpr int SPAN = 3;
+  static_assert(P == 2 && LMAX == 80, "a column of 65..80 levels, two to a group: SPAN warps each");
   int t, c, k, L, bar;
+  int wf;      // first warp of this thread's column
+  int off;     // 1: the column starts inside that warp
   double* scr;   // 2 * SCR doubles
   double* work;  // this column's two work rows (WP doubles each)
   int par;
@@ -487,36 +597,41 @@ struct PackedColumn {
     c = t / L;
     if (c > P) c = P;
     k = t - c * L;
+    const int s0 = min(c, P - 1) * L;
+    wf = s0 >> 5;
+    off = (s0 & 31) != 0;
     scr = scr_grp;
     work = work_grp + (size_t)c * 2 * WP;
     par = 0;
   }
   SHD int w() const { return t >> 5; }
   SHD int lane() const { return t & 31; }
-  SHD int seg0() const { return t - k; }
-  SHD int seglen() const { return (c < P) ? L : T - P * L; }
-  SHD int wfirst() const { return seg0() >> 5; }
-  SHD int wlast() const { return (seg0() + seglen() - 1) >> 5; }
-  // the slot, in a per-warp pair of partials, that holds this segment's
-  // part of warp u (the head partial unless the segment starts inside u)
-  SHD int part(int u) const { return 2 * u + ((u == wfirst() && (seg0() & 31) != 0) ? 1 : 0); }
-  // lanes of this warp in this segment
+  // levels of this thread's column above it in its warp
+  SHD int above() const { return min(lane(), k); }
+  // lanes of this warp in this column (k <= lane: the column starts here)
   SHD unsigned segmask() const {
-    const int w_ = w();
-    const int lo = max(seg0() - 32 * w_, 0), hi = min(seg0() + seglen() - 32 * w_, 32);
-    const unsigned up = (hi >= 32) ? FULLMASK : ((1u << hi) - 1u);
-    return up & ~((1u << lo) - 1u);
+    const unsigned from = k <= lane() ? FULLMASK << (lane() - k) : FULLMASK;
+    const int last = lane() + (c < P ? L - 1 - k : T);  // lane of its last level
+    return last < 31 ? from & ((2u << last) - 1u) : from;
   }
-  // this lane is the last of its segment within its warp
-  SHD bool seg_last_in_warp() const { return lane() == 31 || k == seglen() - 1; }
-  // this lane's segment is the one holding lane 0 of the warp
-  SHD bool in_head() const { return seg0() <= 32 * w(); }
 
   SHD void sync() const { asm volatile("bar.sync %0, %1;" ::"r"(bar), "r"(T) : "memory"); }
   SHD double* slot() {
     double* s = scr + par * SCR;
     par ^= 1;
     return s;
+  }
+  // OR of this column's per-warp words: a pair per warp, of the segment
+  // holding its lane 0 and the one holding its lane 31
+  SHD void put_part(unsigned* s, unsigned bits) const {
+    if (lane() == 0) s[2 * w()] = bits;
+    if (lane() == 31) s[2 * w() + 1] = bits;
+  }
+  SHD unsigned or_parts(const unsigned* s) const {
+    unsigned r = s[2 * wf + off];
+#pragma unroll
+    for (int j = 1; j < SPAN; ++j) r |= s[2 * (wf + j)];
+    return r;
   }
   SHD bool group_any(bool p) {
     unsigned r;
@@ -539,10 +654,50 @@ struct PackedColumn {
     return u;
   }
   template <int N>
-  SHD void prevN(const double (&x)[N], double (&px)[N]) {
+  SHD void nbrsN(const double (&x)[N], double (&xp)[N], double (&xn)[N]) {
+    double* s = slot();
+#pragma unroll
+    for (int n = 0; n < N; ++n) {
+      xp[n] = __shfl_up_sync(FULLMASK, x[n], 1);
+      xn[n] = __shfl_down_sync(FULLMASK, x[n], 1);
+      if (lane() == 0) s[2 * (N * w() + n)] = x[n];
+      if (lane() == 31) s[2 * (N * w() + n) + 1] = x[n];
+    }
+    sync();
+#pragma unroll
+    for (int n = 0; n < N; ++n) {
+      if (lane() == 0 && w() > 0) xp[n] = s[2 * (N * (w() - 1) + n) + 1];
+      if (lane() == 31 && w() < NWG - 1) xn[n] = s[2 * (N * (w() + 1) + n)];
+    }
+  }
+  // the column's any(p), the group's, and x at level k - 1, from one exchange
+  SHD void any_prev(bool p, double x, bool& r, bool& g, double& px) {
+    const unsigned m = __ballot_sync(FULLMASK, p);
+    px = __shfl_up_sync(FULLMASK, x, 1);
+    double* s = slot();
+    unsigned* su = reinterpret_cast<unsigned*>(s + NWG);
+    put_part(su, (m & segmask()) ? 1u : 0u);
+    if (lane() == 31) s[w()] = x;
+    sync();
+    if (lane() == 0 && w() > 0) px = s[w() - 1];
+    r = or_parts(su) != 0;
+    unsigned o = 0;
+#pragma unroll
+    for (int u = 0; u < 2 * NWG; ++u) o |= su[u];
+    g = o != 0;
+  }
+  // the first level of the column where p holds (1 << 30: none) and x at
+  // level k - 1, from one exchange
+  template <int N>
+  SHD int first_prevN(bool p, const double (&x)[N], double (&px)[N]) {
+    const unsigned m = __ballot_sync(FULLMASK, p) & segmask();
 #pragma unroll
     for (int n = 0; n < N; ++n) px[n] = __shfl_up_sync(FULLMASK, x[n], 1);
     double* s = slot();
+    unsigned* su = reinterpret_cast<unsigned*>(s + N * NWG);
+    // 127 less the level, so that the first level is the largest value
+    const unsigned v = m ? 128u - (unsigned)(k - lane() + __ffs(m)) : 0u;
+    put_part(su, v);
     if (lane() == 31) {
 #pragma unroll
       for (int n = 0; n < N; ++n) s[N * w() + n] = x[n];
@@ -552,86 +707,12 @@ struct PackedColumn {
 #pragma unroll
       for (int n = 0; n < N; ++n) px[n] = s[N * (w() - 1) + n];
     }
-  }
-  SHD void nbrs(double x, double& xp, double& xn) {
-    xp = __shfl_up_sync(FULLMASK, x, 1);
-    xn = __shfl_down_sync(FULLMASK, x, 1);
-    double* s = slot();
-    if (lane() == 0) s[2 * w()] = x;
-    if (lane() == 31) s[2 * w() + 1] = x;
-    sync();
-    if (lane() == 0 && w() > 0) xp = s[2 * w() - 1];
-    if (lane() == 31 && w() < NWG - 1) xn = s[2 * w() + 2];
-  }
-  // ------------------------------------------------ column reductions
-  SHD bool any(bool p) {
-    unsigned m[1] = {p ? 1u : 0u};
-    anyN<1>(m);
-    return m[0] != 0;
-  }
-  SHD void any3(bool a, bool b, bool c3, bool& ra, bool& rb, bool& rc) {
-    unsigned m[3] = {a ? 1u : 0u, b ? 1u : 0u, c3 ? 1u : 0u};
-    anyN<3>(m);
-    ra = m[0] != 0;
-    rb = m[1] != 0;
-    rc = m[2] != 0;
-  }
-  // the column's any() and, from the same exchange, the group's (every
-  // warp's parts ORed)
-  SHD bool any_group(bool p, bool& g) {
-    unsigned m[1] = {p ? 1u : 0u}, gm = 0;
-    anyN<1>(m, &gm);
-    g = gm != 0;
-    return m[0] != 0;
-  }
-  SHD void any3_group(bool a, bool b, bool c3, bool& ra, bool& rb, bool& rc, bool& ga, bool& gb, bool& gc) {
-    unsigned m[3] = {a ? 1u : 0u, b ? 1u : 0u, c3 ? 1u : 0u}, gm = 0;
-    anyN<3>(m, &gm);
-    ra = m[0] != 0;
-    rb = m[1] != 0;
-    rc = m[2] != 0;
-    ga = (gm & 1u) != 0;
-    gb = (gm & 2u) != 0;
-    gc = (gm & 4u) != 0;
-  }
-  template <int N>
-  SHD void anyN(unsigned (&m)[N], unsigned* group = nullptr) {
-    const unsigned sm_ = segmask();
-    unsigned bits = 0;
+    unsigned f = su[2 * wf + off];
 #pragma unroll
-    for (int n = 0; n < N; ++n) bits |= ((__ballot_sync(FULLMASK, m[n] != 0) & sm_) != 0u ? 1u : 0u) << n;
-    unsigned* s = reinterpret_cast<unsigned*>(slot());
-    if (lane() == 0) s[2 * w()] = bits;
-    if (lane() == 31) s[2 * w() + 1] = bits;
-    sync();
-    unsigned r = 0;
-    for (int u = wfirst(); u <= wlast(); ++u) r |= s[part(u)];
-    if (group) {
-      unsigned gr = 0;
-#pragma unroll
-      for (int u = 0; u < NWG; ++u) gr |= s[2 * u] | s[2 * u + 1];
-      *group = gr;
-    }
-#pragma unroll
-    for (int n = 0; n < N; ++n) m[n] = (r >> n) & 1u;
+    for (int j = 1; j < SPAN; ++j) f = max(f, su[2 * (wf + j)]);
+    return f ? 127 - (int)f : 1 << 30;
   }
-  SHD int min_int(int v) {
-    // segmented inclusive min-scan down the warp, then the per-warp parts
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-      const int o = __shfl_up_sync(FULLMASK, v, d);
-      if (lane() >= d && k >= d) v = min(v, o);
-    }
-    int* s = reinterpret_cast<int*>(slot());
-    if (lane() == 31) s[2 * w() + 1] = v;
-    if (in_head() && seg_last_in_warp()) s[2 * w()] = v;
-    sync();
-    int m = s[part(wfirst())];
-    for (int u = wfirst() + 1; u <= wlast(); ++u) m = min(m, s[part(u)]);
-    return m;
-  }
-  // values of N fields at level k0 of this column (the idle tail reads the
-  // last column's)
+  // values of N fields at level k0 of this column
   template <int N>
   SHD void bcastN(const double (&x)[N], int k0, double (&x0)[N]) {
     double* s = slot();
@@ -651,36 +732,37 @@ struct PackedColumn {
     x0 = r[0];
     y0 = r[1];
   }
-  SHD double bcast(double x, int k0) {
-    const double v[1] = {x};
-    double r[1];
-    bcastN<1>(v, k0, r);
-    return r[0];
-  }
   // ------------------------------------------------ recurrences
   // N independent top-down affine scans X_k = a_k + b_k X_{k-1} (b must
-  // vanish at k = 0)
+  // vanish at k = 0), their values at level k - 1, and the column's any() of
+  // N flags, from one exchange
   template <int N>
-  SHD void scanN(const double (&a)[N], const double (&b)[N], double (&x)[N]) {
+  SHD void scanN_prev_any(const double (&a)[N], const double (&b)[N], bool (&p)[N], double (&x)[N], double (&xp)[N]) {
     double A[N], B[N];
+    unsigned bits = 0;
+    const unsigned seg = segmask();
 #pragma unroll
     for (int n = 0; n < N; ++n) {
       A[n] = a[n];
       B[n] = b[n];
+      bits |= ((__ballot_sync(FULLMASK, p[n]) & seg) != 0u ? 1u : 0u) << n;
     }
+    const int up = above();
 #pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
 #pragma unroll
       for (int n = 0; n < N; ++n) {
         const double pA = __shfl_up_sync(FULLMASK, A[n], d);
         const double pB = __shfl_up_sync(FULLMASK, B[n], d);
-        if (lane() >= d && k >= d) {
+        if (up >= d) {
           A[n] = A[n] + B[n] * pA;
           B[n] = B[n] * pB;
         }
       }
     }
     double* s = slot();
+    unsigned* su = reinterpret_cast<unsigned*>(s + 2 * N * NWG);
+    put_part(su, bits);
     if (lane() == 31) {
 #pragma unroll
       for (int n = 0; n < N; ++n) {
@@ -689,44 +771,59 @@ struct PackedColumn {
       }
     }
     sync();
-    // the carry from this column's earlier warps (lane 31 of each is in it)
+    // the carry from this column's earlier warps, at most SPAN - 1 (lane 31 of each is in it)
 #pragma unroll
     for (int n = 0; n < N; ++n) {
       double X = 0.0;
-      for (int u = wfirst(); u < w(); ++u) X = s[2 * N * u + 2 * n] + s[2 * N * u + 2 * n + 1] * X;
-      x[n] = (w() > wfirst()) ? A[n] + B[n] * X : A[n];
+#pragma unroll
+      for (int j = 0; j < SPAN - 1; ++j)
+        if (wf + j < w()) X = s[2 * N * (wf + j) + 2 * n] + s[2 * N * (wf + j) + 2 * n + 1] * X;
+      x[n] = (w() > wf) ? A[n] + B[n] * X : A[n];
+      const double v = __shfl_up_sync(FULLMASK, x[n], 1);
+      xp[n] = lane() > 0 ? v : X;
     }
+    bits = or_parts(su);
+#pragma unroll
+    for (int n = 0; n < N; ++n) p[n] = (bits >> n) & 1u;
   }
   SHD double scan_affine(double a, double b) {
     const double aa[1] = {a}, bb[1] = {b};
-    double xx[1];
-    scanN<1>(aa, bb, xx);
+    double xx[1], xp[1];
+    bool p[1] = {false};
+    scanN_prev_any<1>(aa, bb, p, xx, xp);
     return xx[0];
   }
   SHD void scan_affine2(double a1, double b1, double a2, double b2, double& x1, double& x2) {
     const double aa[2] = {a1, a2}, bb[2] = {b1, b2};
-    double xx[2];
-    scanN<2>(aa, bb, xx);
+    double xx[2], xp[2];
+    bool p[2] = {false, false};
+    scanN_prev_any<2>(aa, bb, p, xx, xp);
     x1 = xx[0];
     x2 = xx[1];
   }
   // layer thickness from the BACKWARD height sweep:
   // ze_k = zs + sum_{j >= k} (-dz1_j); dz_k = ze_k - ze_{k+1}, dz_{L-1} = ze_{L-1} - zs
   SHD double heights(double x, double zs) {
+    const int below = min(31 - lane(), (c < P ? L : T - P * L) - 1 - k);  // levels of the column below in the warp
 #pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
       const double v = __shfl_down_sync(FULLMASK, x, d);
-      if (lane() + d < 32 && k + d < seglen()) x = x + v;
+      if (below >= d) x = x + v;
     }
     double zn_in_warp = __shfl_down_sync(FULLMASK, x, 1);  // suffix at k + 1 within the warp
     double* s = slot();
     // lane 0 of each of this column's later warps holds that warp's part
     if (lane() == 0) s[w()] = x;
     sync();
+    const int wl = wf + SPAN - 1;
     double cc = 0.0, cn = 0.0;
-    for (int u = wlast(); u > w(); --u) cc = cc + s[u];
-    if (lane() == 31 && w() < wlast()) {
-      for (int u = wlast(); u > w() + 1; --u) cn = cn + s[u];
+#pragma unroll
+    for (int j = 0; j < SPAN - 1; ++j)
+      if (wl - j > w()) cc = cc + s[wl - j];
+    if (lane() == 31 && w() < wl) {
+#pragma unroll
+      for (int j = 0; j < SPAN - 2; ++j)
+        if (wl - j > w() + 1) cn = cn + s[wl - j];
       zn_in_warp = s[w() + 1];
     }
     const double ze = zs + (x + cc);
@@ -745,21 +842,26 @@ struct PackedColumn {
 // the mass leaving the bottom of level k. The telescoped form is used here.
 // It equals the running sum in exact arithmetic, but it does not cancel: the
 // running sum loses all its digits when little mass reaches the ground.
+//
+// vtp: the fall speed at the level above; fp: the flux there (the same
+// product that level forms).
 template <class Col>
-SHD double implicit_fall(Col& C, double& q, double vt, double dz, double dp1, bool valid, double dtf) {
-  const double dd = dtf * vt;
+SHD double implicit_fall(Col& C, double& q, double vt, double vtp, double dz, double dp1, bool valid, double dtf,
+                         double& fp) {
+  const double dd = dtf * vt, ddp = dtf * vtp;
   const double qmass = valid ? q * dp1 : 0.0;
-  const double ddp = C.prev(dd);
   const Divisor<double> by_D(dz + dd);
-  double a = by_D(qmass);
-  double b = (C.k == 0) ? 0.0 : by_D(ddp);
+  double a[1] = {by_D(qmass)}, b[1] = {(C.k == 0) ? 0.0 : by_D(ddp)};
   if (!valid) {
-    a = 0.0;
-    b = 0.0;
+    a[0] = 0.0;
+    b[0] = 0.0;
   }
-  const double r = C.scan_affine(a, b);
-  if (valid) q = qdiv(r * dz, dp1);
-  return valid ? dd * r : 0.0;
+  double r[1], rp[1];
+  bool p[1] = {false};
+  C.template scanN_prev_any<1>(a, b, p, r, rp);
+  fp = valid ? ddp * rp[0] : 0.0;
+  if (valid) q = qdiv(r[0] * dz, dp1);
+  return valid ? dd * r[0] : 0.0;
 }
 
 // Implicit heating by falling condensate (microphysics.py:516-557 with
@@ -797,10 +899,11 @@ SHD double w_update(int k, double w, double dm, double flux, double vt, double f
 // 1341-1367), before the h_var floor: dq_k = 0.5 (q_k - q_{k-1}).
 template <class Col>
 SHD double mono_slope(Col& C, double q) {
-  double qp, qn;
-  C.nbrs(q, qp, qn);
-  const double dq = 0.5 * (q - qp);
-  const double dqn = 0.5 * (qn - q);
+  const double x[1] = {q};
+  double xp[1], xn[1];
+  C.template nbrsN<1>(x, xp, xn);
+  const double dq = 0.5 * (q - xp[0]);
+  const double dqn = 0.5 * (xn[0] - q);
   double v = 0.0;
   if (C.k >= 1 && C.k <= C.L - 2) {
     v = 0.5 * qmin(fabs(dq + dqn), 0.5 * q);
@@ -1049,14 +1152,19 @@ SHD void fields_init(Col& C, const MpConst& K, bool valid, double pt, double qvi
       if (valid) S.qv = wq[k];
     }
     if (k < L - 1 && S.qv < 0.0) S.qv = 0.0;
-    // bottom layer borrows from the layer above (:253-276)
-    double qb, db, qb1, db1;
-    C.bcast2(S.qv, P.dp1, L - 1, qb, db);
-    C.bcast2(S.qv, P.dp1, L - 2, qb1, db1);
-    if ((qb < 0.0) && (qb1 > 0.0)) {
-      const double dq = qmin(-qb * db, qb1 * db1);
-      if (k == L - 2) S.qv = S.qv - qdiv(dq, P.dp1);
-      if (k == L - 1) S.qv = S.qv + qdiv(dq, P.dp1);
+    // bottom layer borrows from the layer above (:253-276): the two levels
+    // form the same dq
+    const double x[2] = {S.qv, P.dp1};
+    double xp[2], xn[2];
+    C.template nbrsN<2>(x, xp, xn);
+    if (k == L - 2 || k == L - 1) {
+      const bool bot = k == L - 1;
+      const double qb = bot ? S.qv : xn[0], db = bot ? P.dp1 : xn[1];
+      const double qb1 = bot ? xp[0] : S.qv, db1 = bot ? xp[1] : P.dp1;
+      if ((qb < 0.0) && (qb1 > 0.0)) {
+        const double dq = qdiv(qmin(-qb * db, qb1 * db1), P.dp1);
+        S.qv = bot ? S.qv + dq : S.qv - dq;
+      }
     }
   }
 }
@@ -1084,46 +1192,48 @@ struct NoRec {
 
 // warm_rain (:280-653) after the geometry: rain evaporation and accretion,
 // implicit rain fall with the vertical-velocity transport and heating, then
-// autoconversion. Returns the rain flux m1_rain at this level and the
-// surface flux r1.
+// autoconversion. Returns the rain flux m1_rain at this level (at the bottom
+// level: the surface flux) and m1_prev, the flux at the level above.
 // A recorder gets the states after the first evaporation (slot 0), after the
 // fall (1) and after the second evaporation (2), the liquid slope (value 0)
 // and the column's rain-fall decision.
 template <bool MIXED, class Col, class Rec = NoRec>
 SHD void warm_rain(Col& C, const MpConst& K, const MpConstF& KF, bool valid, LevState& S, const StepGeom& P,
-                   double& vtr, double& m1_rain, double& r1, bool* falls = nullptr, const Rec& rec = Rec()) {
-  const int k = C.k, L = C.L;
+                   double& vtr, double& m1_rain, double& m1_prev, bool* falls = nullptr, const Rec& rec = Rec()) {
+  const int k = C.k;
   double &qv = S.qv, &ql = S.ql, &qr = S.qr, &qi = S.qi, &qs = S.qs, &qg = S.qg, &tz = S.tz, &w = S.w;
   const double dt5 = 0.5 * K.dt_rain;
   m1_rain = 0.0;
-  bool gfall;
-  const bool fall = C.any_group(valid && (qr > QRMIN), gfall);
+  m1_prev = 0.0;
+  // the fall speed before it is known whether the column's rain falls (it is
+  // VR_MIN without a test of more than qr where none does), so that the
+  // decision and the speed above come from one exchange
+  double vt, vp;
+  if constexpr (MIXED)
+    vt = rain_fspeed_m(K, qr, P.den);
+  else
+    vt = rain_fspeed(K, qr, P.den);
+  bool fall, gfall;
+  C.any_prev(valid && (qr > QRMIN), vt, fall, gfall, vp);
   if (falls) *falls = fall;
   rec.flag(fall);
-  r1 = 0.0;
-  if (!fall) vtr = VF_MIN;
+  vtr = fall ? vt : VF_MIN;
   // The fall's vertical operations run whenever a column sharing the
   // barrier has falling rain; a column without it takes part with no mass
   // (valid false), which leaves its state unchanged and its flux zero.
   if (gfall) {
     const bool vf = valid && fall;
     if (fall) {
-      if constexpr (MIXED) {
-        vtr = rain_fspeed_m(K, qr, P.den);
+      if constexpr (MIXED)
         revap_racc_m(K, KF, dt5, P.h_var, qg, qi, ql, qr, qs, qv, tz, P.den, P.denfac);
-      } else {
-        vtr = rain_fspeed(K, qr, P.den);
+      else
         revap_racc(K, dt5, P.h_var, qg, qi, ql, qr, qs, qv, tz, P.den, P.denfac);
-      }
     }
     rec.state(0, S);
     const double dm = P.dp1 * (1.0 + qv + ql + qr + qi + qs + qg);
-    m1_rain = implicit_fall(C, qr, vtr, P.dz, P.dp1, vf, K.dt_rain);
-    double fv[2] = {m1_rain, vtr}, pv[2];
-    C.template prevN<2>(fv, pv);
-    r1 = C.bcast(m1_rain, L - 1);
-    if (fall && K.do_sedi_w) w = w_update(k, w, dm, m1_rain, vtr, pv[0], pv[1]);
-    if (K.do_sedi_heat) sedi_heat(C, K, tz, P.dz1, P.dp1, qv, ql, qr, qi, qs, qg, m1_rain, pv[0], vf, K.C_LIQ);
+    m1_rain = implicit_fall(C, qr, vtr, vp, P.dz, P.dp1, vf, K.dt_rain, m1_prev);
+    if (fall && K.do_sedi_w) w = w_update(k, w, dm, m1_rain, vtr, m1_prev, vp);
+    if (K.do_sedi_heat) sedi_heat(C, K, tz, P.dz1, P.dp1, qv, ql, qr, qi, qs, qg, m1_rain, m1_prev, vf, K.C_LIQ);
     rec.state(1, S);
     if (fall) {
       if constexpr (MIXED)
@@ -1161,12 +1271,13 @@ SHD void warm_rain(Col& C, const MpConst& K, const MpConstF& KF, bool valid, Lev
 // sedimentation (:657-1217): fall speeds, cloud ice melting, and the
 // implicit falls of ice, snow and graupel with their vertical-velocity
 // transport and heating. Returns the solid flux m1_sol at this level and
-// adds the surface fluxes to ice, snow and graupel.
-// A recorder gets the cloud ice fall speed (value 0).
+// m1_prev, the one at the level above; the bottom level adds the surface
+// fluxes to ice, snow and graupel. A recorder gets the cloud ice fall speed
+// (value 0).
 template <bool MIXED, class Col, class Rec = NoRec>
 SHD void sedimentation(Col& C, const MpConst& K, const MpConstF& KF, bool valid, LevState& S,
-                       const StepGeom& P, double& vtg, double& vts, double& m1_sol, double& ice, double& snow,
-                       double& graupel, unsigned* flags = nullptr, const Rec& rec = Rec()) {
+                       const StepGeom& P, double& vtg, double& vts, double& m1_sol, double& m1_prev, double& ice,
+                       double& snow, double& graupel, unsigned* flags = nullptr, const Rec& rec = Rec()) {
   const int k = C.k, L = C.L;
   double &qv = S.qv, &ql = S.ql, &qr = S.qr, &qi = S.qi, &qs = S.qs, &qg = S.qg, &tz = S.tz, &w = S.w;
   const double dp1 = P.dp1, dz = P.dz;
@@ -1177,76 +1288,77 @@ SHD void sedimentation(Col& C, const MpConst& K, const MpConstF& KF, bool valid,
     fall_speed(K, qg, qi, qs, tz, P.den, vtg, vti, vts);
   rec.value(0, vti);
   m1_sol = 0.0;
-  // cloud ice melting at and below the first level warmer than tice (:702-746)
-  const int first = C.min_int((valid && tz > K.tice) ? k : (1 << 30));
+  m1_prev = 0.0;
+  // cloud ice melting at and below the first level warmer than tice (:702-746);
+  // the fall speeds above come with the same exchange
+  const double vt[3] = {vti, vts, vtg};
+  double vp[3];
+  const int first = C.template first_prevN<3>(valid && tz > K.tice, vt, vp);
   if ((k >= first || k == L - 1) && valid) sedi_ice_melt(K, qv, ql, qr, qi, qs, qg, tz);
   // ice (:773-900), snow (:902-1035) and graupel (:1037-1168): their
-  // implicit falls are independent of one another, so the three share
-  // each column exchange; the vertical-velocity updates, which the
-  // reference applies species after species, stay in that order.
-  bool fi, fs, fg, gi, gs, gg;
-  C.any3_group(valid && (qi > QRMIN), valid && (qs > QRMIN), valid && (qg > QRMIN), fi, fs, fg, gi, gs, gg);
-  fi = fi && (K.vi_fac >= 1.0e-5);
-  gi = gi && (K.vi_fac >= 1.0e-5);
+  // implicit falls are independent of one another, so the three share one
+  // exchange, which also decides which of them fall (in nearly every column
+  // of weather some does; a column where none does scans zeros); the
+  // vertical-velocity updates, which the reference applies species after
+  // species, stay in that order.
+  bool f[3] = {valid && (qi > QRMIN), valid && (qs > QRMIN), valid && (qg > QRMIN)};
+  double dd[3], ddp[3];
+#pragma unroll
+  for (int n = 0; n < 3; ++n) {
+    dd[n] = K.dts * vt[n];
+    ddp[n] = K.dts * vp[n];
+  }
+  const double qq[3] = {qi, qs, qg};
+  double ra[3], rb[3], r[3], rp[3];
+#pragma unroll
+  for (int n = 0; n < 3; ++n) {
+    const double qmass = valid ? qq[n] * dp1 : 0.0;
+    const Divisor<double> by_D(dz + dd[n]);
+    ra[n] = by_D(qmass);
+    rb[n] = (k == 0) ? 0.0 : by_D(ddp[n]);
+    if (!valid) {
+      ra[n] = 0.0;
+      rb[n] = 0.0;
+    }
+  }
+  C.template scanN_prev_any<3>(ra, rb, f, r, rp);
+  const bool fi = f[0] && (K.vi_fac >= 1.0e-5), fs = f[1], fg = f[2];
   if (flags)
     *flags |= (fi ? FLAG_ICE_FALLS : 0u) | (fs ? FLAG_SNOW_FALLS : 0u) | (fg ? FLAG_GRAUPEL_FALLS : 0u) |
               ((unsigned)min(first, L - 1) << FLAG_MELT_SHIFT);
-  double mp = 0.0;  // m1_sol at the level above, for the heating
-  // taken by every column sharing the barrier when one of them has a
-  // falling species; each species' results apply only where it falls
-  if (gi || gs || gg) {
-    const double dd[3] = {K.dts * vti, K.dts * vts, K.dts * vtg};
-    double ddp[3];
-    C.template prevN<3>(dd, ddp);
-    const double qq[3] = {qi, qs, qg};
-    double ra[3], rb[3], r[3];
+  double flux[3], fp[3];  // of each species, here and at the level above
 #pragma unroll
-    for (int n = 0; n < 3; ++n) {
-      const double qmass = valid ? qq[n] * dp1 : 0.0;
-      const Divisor<double> by_D(dz + dd[n]);
-      ra[n] = by_D(qmass);
-      rb[n] = (k == 0) ? 0.0 : by_D(ddp[n]);
-      if (!valid) {
-        ra[n] = 0.0;
-        rb[n] = 0.0;
-      }
-    }
-    C.template scanN<3>(ra, rb, r);
-    double flux[3];
-#pragma unroll
-    for (int n = 0; n < 3; ++n) flux[n] = valid ? dd[n] * r[n] : 0.0;
-    const Divisor<double> by_dp1(dp1);
-    const double dm_i = dp1 * (1.0 + qv + ql + qr + qi + qs + qg);
-    if (fi && valid) qi = by_dp1(r[0] * dz);
-    const double dm_s = dp1 * (1.0 + qv + ql + qr + qi + qs + qg);
-    if (fs && valid) qs = by_dp1(r[1] * dz);
-    const double dm_g = dp1 * (1.0 + qv + ql + qr + qi + qs + qg);
-    if (fg && valid) qg = by_dp1(r[2] * dz);
-    double sfc[3];
-    C.template bcastN<3>(flux, L - 1, sfc);
-    const double nv[6] = {flux[0], vti, flux[1], vts, flux[2], vtg};
-    double pv[6];
-    C.template prevN<6>(nv, pv);
-    if (fi) {
-      m1_sol = flux[0];
-      mp = pv[0];
-      if (K.do_sedi_w) w = w_update(k, w, dm_i, flux[0], vti, pv[0], pv[1]);
-      ice = ice + sfc[0];
-    }
-    if (fs) {
-      m1_sol = m1_sol + flux[1];
-      mp = mp + pv[2];
-      if (K.do_sedi_w) w = w_update(k, w, dm_s, flux[1], vts, pv[2], pv[3]);
-      snow = snow + sfc[1];
-    }
-    if (fg) {
-      m1_sol = m1_sol + flux[2];
-      mp = mp + pv[4];
-      if (K.do_sedi_w) w = w_update(k, w, dm_g, flux[2], vtg, pv[4], pv[5]);
-      graupel = graupel + sfc[2];
-    }
+  for (int n = 0; n < 3; ++n) {
+    flux[n] = valid ? dd[n] * r[n] : 0.0;
+    fp[n] = valid ? ddp[n] * rp[n] : 0.0;
   }
-  if (K.do_sedi_heat) sedi_heat(C, K, tz, P.dz1, dp1, qv, ql, qr, qi, qs, qg, m1_sol, mp, valid, K.C_ICE);
+  const Divisor<double> by_dp1(dp1);
+  const double dm_i = dp1 * (1.0 + qv + ql + qr + qi + qs + qg);
+  if (fi && valid) qi = by_dp1(r[0] * dz);
+  const double dm_s = dp1 * (1.0 + qv + ql + qr + qi + qs + qg);
+  if (fs && valid) qs = by_dp1(r[1] * dz);
+  const double dm_g = dp1 * (1.0 + qv + ql + qr + qi + qs + qg);
+  if (fg && valid) qg = by_dp1(r[2] * dz);
+  const bool bottom = k == L - 1;
+  if (fi) {
+    m1_sol = flux[0];
+    m1_prev = fp[0];
+    if (K.do_sedi_w) w = w_update(k, w, dm_i, flux[0], vti, fp[0], vp[0]);
+    if (bottom) ice = ice + flux[0];
+  }
+  if (fs) {
+    m1_sol = m1_sol + flux[1];
+    m1_prev = m1_prev + fp[1];
+    if (K.do_sedi_w) w = w_update(k, w, dm_s, flux[1], vts, fp[1], vp[1]);
+    if (bottom) snow = snow + flux[1];
+  }
+  if (fg) {
+    m1_sol = m1_sol + flux[2];
+    m1_prev = m1_prev + fp[2];
+    if (K.do_sedi_w) w = w_update(k, w, dm_g, flux[2], vtg, fp[2], vp[2]);
+    if (bottom) graupel = graupel + flux[2];
+  }
+  if (K.do_sedi_heat) sedi_heat(C, K, tz, P.dz1, dp1, qv, ql, qr, qi, qs, qg, m1_sol, m1_prev, valid, K.C_ICE);
 }
 
 // icloud (:1220-1449): instant melting or freezing, the ice slope, the ice
@@ -1314,7 +1426,8 @@ SHD void mp_body(const MpArgs& A, double* sm, double* scr, double* work, const i
   LevState S;
   StepGeom P;
   double qa = valid ? TL(IN_QAZ) : 0.0;
-  double m1 = 0.0, m1_sol = 0.0, vtr = VF_MIN, vtg = VF_MIN, vts = VF_MIN;
+  // the precipitation flux summed over the sub-steps, here and at the level above
+  double m1 = 0.0, mp = 0.0, m1_sol = 0.0, mp_sol = 0.0, vtr = VF_MIN, vtg = VF_MIN, vts = VF_MIN;
   P.den = 1.0;
   P.denfac = 1.0;
   P.dz1 = -100.0;
@@ -1335,15 +1448,16 @@ SHD void mp_body(const MpArgs& A, double* sm, double* scr, double* work, const i
     for (int pass = 0; pass < 2; ++pass) {
       const bool is_first = pass == 0;
       if (is_first) substep_geometry(C, K, valid, valid ? TL(IN_PT) : 250.0, valid ? TL(IN_DELZ) : -100.0, S, P);
-      double m1_rain, r1;
+      double m1_rain, mp_rain;
       bool falls = false;
-      warm_rain<MIXED>(C, K, KF, valid, S, P, vtr, m1_rain, r1, FLAGS ? &falls : nullptr);
+      warm_rain<MIXED>(C, K, KF, valid, S, P, vtr, m1_rain, mp_rain, FLAGS ? &falls : nullptr);
       if constexpr (FLAGS) fl |= falls ? (is_first ? FLAG_RAIN_FALLS_1 : FLAG_RAIN_FALLS_2) : 0u;
-      rain = rain + r1;
+      if (k == L - 1) rain = rain + m1_rain;
       m1 = is_first ? m1 + m1_rain : m1 + m1_rain + m1_sol;
+      mp = is_first ? mp + mp_rain : mp + mp_rain + mp_sol;
       if (!is_first) break;
-      sedimentation<MIXED>(C, K, KF, valid, S, P, vtg, vts, m1_sol, ice, snow, graupel, FLAGS ? &fl : nullptr);
-      rain = rain + 0.0;
+      sedimentation<MIXED>(C, K, KF, valid, S, P, vtg, vts, m1_sol, mp_sol, ice, snow, graupel,
+                           FLAGS ? &fl : nullptr);
     }
     icloud<MIXED>(C, K, KF, valid, S, P, qa, vtg, vtr, vts);
     if constexpr (FLAGS) {
@@ -1358,7 +1472,6 @@ SHD void mp_body(const MpArgs& A, double* sm, double* scr, double* work, const i
   const double v0 = valid ? TL(IN_VA) : 0.0;
   double u1 = u0, v1 = v0;
   if (K.sedi_transport) {
-    const double mp = C.prev(m1);
     double au, av, b;
     if (k == 0 || !valid) {
       au = u0;
@@ -1409,7 +1522,7 @@ SHD void mp_body(const MpArgs& A, double* sm, double* scr, double* work, const i
                    isfinite(inc_u) && isfinite(inc_v) && isfinite(w) && isfinite(qa)))
       atomicCAS(A.err, 0, (int)(col + 1));
   }
-  if (k == 0 && col_ok) {
+  if (k == L - 1 && col_ok) {
     const double convt = 86400.0 * K.rdt * K.RGRAV;
     if (A.rain) A.rain[col] = rain * convt;
     if (A.snow) A.snow[col] = snow * convt;

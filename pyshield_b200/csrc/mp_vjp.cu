@@ -904,8 +904,8 @@ __global__ void __launch_bounds__(LY::THREADS, MINB) vjp_replay_kernel(const __g
     W.sc(SC_CCN)[cc] = P.ccn;
     W.sc(SC_CPRAUT)[cc] = P.c_praut;
   }
-  double m1 = 0.0, m1_sol = 0.0, vtr = VF_MIN, vtg = VF_MIN, vts = VF_MIN, qa = 0.0, ice = 0.0, snow = 0.0,
-         graupel = 0.0;
+  double m1 = 0.0, m1_sol = 0.0, mp_sol = 0.0, vtr = VF_MIN, vtg = VF_MIN, vts = VF_MIN, qa = 0.0, ice = 0.0,
+         snow = 0.0, graupel = 0.0;
   constexpr int NREC = SM::NREC;
   constexpr int64_t RS = (int64_t)G * RP;  // stride between record tiles
   const double* rec = sm + SM::rec;
@@ -935,9 +935,9 @@ __global__ void __launch_bounds__(LY::THREADS, MINB) vjp_replay_kernel(const __g
     // the warm_rain code, run twice, as in the forward kernel)
 #pragma unroll 1
     for (int pass = 0; pass < 2; ++pass) {
-      double m1r, r1;
+      double m1r, mpr;
       // tiles 0 .. 12: the pass's block; 13: the fall speed; 14: the slope
-      warm_rain<false>(C, K, KF, valid, S, P, vtr, m1r, r1, nullptr,
+      warm_rain<false>(C, K, KF, valid, S, P, vtr, m1r, mpr, nullptr,
                        VjpRec{rt, rt + 14 * RS, W.scc(it, pass ? SCC_FALL_B : SCC_FALL_A) + cc, RS, valid, head,
                               false});
       m1 = (pass == 0) ? m1 + m1r : m1 + m1r + m1_sol;
@@ -953,7 +953,7 @@ __global__ void __launch_bounds__(LY::THREADS, MINB) vjp_replay_kernel(const __g
       }
       if (pass == 1) break;
       // tiles 0 .. 7: the state after sedimentation; 8, 9, 10: vtg, vts, vti
-      sedimentation<false>(C, K, KF, valid, S, P, vtg, vts, m1_sol, ice, snow, graupel, nullptr,
+      sedimentation<false>(C, K, KF, valid, S, P, vtg, vts, m1_sol, mp_sol, ice, snow, graupel, nullptr,
                            VjpRec{nullptr, rt + 10 * RS, nullptr, RS, valid, false, false});
       put_lev(0, S);
       put(8, vtg);
