@@ -122,6 +122,7 @@ int step_impl(Handle* h, const ShieldMpFields* F, double timestep, int precision
     if (set_timestep(h->cfg, K2, timestep, why) != SHIELD_OK) return fail(h, SHIELD_EINVAL, why);
     h->K = K2;
   }
+  if (h->ncol > INT32_MAX) return fail(h, SHIELD_ELAYOUT, "more than 2^31 - 1 columns");
   const ShieldField3D* ins[] = {&F->pt, &F->qvapor, &F->qliquid, &F->qrain, &F->qice, &F->qsnow, &F->qgraupel,
                                 &F->qcld, &F->ua, &F->va, &F->delprsi, &F->delz, &F->wmp};
   const ShieldField3D* outs[] = {&F->pt_dt, &F->qv_dt, &F->ql_dt, &F->qr_dt, &F->qi_dt,
@@ -162,6 +163,7 @@ int step_impl(Handle* h, const ShieldMpFields* F, double timestep, int precision
                       std::to_string((int64_t)h->K.ntimes * h->ncol));
     A.flags = flags;
   }
+  plan_layout(A);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   cudaError_t e = cudaSuccess;
   if (h->K.de_ice) {
@@ -413,7 +415,7 @@ extern "C" int shield_mp_ensemble_create(const ShieldMpConfig* cfg, int nz, int 
   setupm(*cfg, base);
   for (int m = 0; m < nm; ++m) {
     const ShieldMpMember& M = mem[m];
-    if (M.nx < 1 || M.ny < 1 || !M.area.ptr) {
+    if (M.nx < 1 || M.ny < 1 || !M.area.ptr || (int64_t)M.nx * M.ny > INT32_MAX) {
       plan_free(p);
       return fail(nullptr, SHIELD_EINVAL, "member " + std::to_string(m) + ": bad domain or area");
     }
@@ -480,6 +482,7 @@ extern "C" int shield_mp_ensemble_create(const ShieldMpConfig* cfg, int nz, int 
     const Fld3 qaz{p->d_qaz + p->qaz_off[m], 1, A.nx, A.ncol};
     A.in[IN_QAZ] = qaz;
     A.out[OUT_QAZ] = qaz;
+    plan_layout(A);
     e = mp_gather_area(mem[m].area.ptr, mem[m].area.si, mem[m].area.sj, A.nx, A.ny, p->d_area + area_off[m]);
     if (e != cudaSuccess) break;
   }
@@ -654,6 +657,7 @@ extern "C" int shield_mp_step_noalloc(const ShieldMpConfig* cfg, int nx, int ny,
   A.ice = F->ice;
   A.graupel = F->graupel;
   A.err = reinterpret_cast<int*>(scratch + kNoAllocMaxCells);
+  plan_layout(A);
   // The array keeps whatever the last call on this device left in it. The
   // first step of a run (or of another domain) starts from a zero
   // accumulator and a clear error word, as a freshly constructed handle does.

@@ -46,8 +46,10 @@ template <int NW>
 struct Column {
   static constexpr int WP = Tiles<NW>::RP;  // pitch of the work rows
   int w, lane, k, L, bar;
+  static constexpr int CV = 10;  // doubles of the column's own values
   double* scr;   // 2 * SCR doubles
   double* work;  // 2 * RP doubles, for the sequential vapour borrow
+  double* cv;    // CV doubles
   int par;
 
   SHD void sync() const { asm volatile("bar.sync %0, %1;" ::"r"(bar), "r"(32 * NW) : "memory"); }
@@ -585,11 +587,13 @@ struct PackedColumn {
   int t, c, k, L, bar;
   int wf;      // first warp of this thread's column
   int off;     // 1: the column starts inside that warp
+  static constexpr int CV = 10;  // doubles of a column's own values
   double* scr;   // 2 * SCR doubles
   double* work;  // this column's two work rows (WP doubles each)
+  double* cv;    // and its CV doubles
   int par;
 
-  // scr_grp / work_grp: the group's scratch and its (P + 1) x 2 work rows
+  // scr_grp / work_grp: the group's scratch and its P + 1 columns' work rows and values
   SHD void init(int t_, int L_, int bar_, double* scr_grp, double* work_grp) {
     t = t_;
     L = L_;
@@ -601,7 +605,8 @@ struct PackedColumn {
     wf = s0 >> 5;
     off = (s0 & 31) != 0;
     scr = scr_grp;
-    work = work_grp + (size_t)c * 2 * WP;
+    work = work_grp + (size_t)c * (2 * WP + CV);
+    cv = work + 2 * WP;
     par = 0;
   }
   SHD int w() const { return t >> 5; }
@@ -933,7 +938,7 @@ struct ColumnLayout {
   static constexpr int THREADS = 32 * NW * G_;
   static constexpr int RP = Tiles<NW>::RP;
   static constexpr int SCR = Tiles<NW>::SCR;
-  static constexpr int WORK = 2 * RP;
+  static constexpr int WORK = 2 * RP + Col::CV;
   // set up thread tid's column object; returns its block column (G: none)
   static SHD int setup(Col& C, int tid, int L, double* scr, double* work) {
     const int g = tid / (32 * NW);
@@ -944,6 +949,7 @@ struct ColumnLayout {
     C.bar = 1 + g;
     C.scr = scr + (size_t)g * 2 * SCR;
     C.work = work + (size_t)g * WORK;
+    C.cv = C.work + 2 * RP;
     C.par = 0;
     return g;
   }
@@ -959,7 +965,7 @@ struct PackedLayout {
   static constexpr int THREADS = 32 * NWG * NGRP_;
   static constexpr int RP = Col::WP;
   static constexpr int SCR = Col::SCR;
-  static constexpr int WORK = (P + 1) * 2 * Col::WP;
+  static constexpr int WORK = (P + 1) * (2 * Col::WP + Col::CV);
   static SHD int setup(Col& C, int tid, int L, double* scr, double* work) {
     const int gi = tid / (32 * NWG);
     C.init(tid % (32 * NWG), L, 1 + gi, scr + (size_t)gi * 2 * SCR, work + (size_t)gi * WORK);
@@ -986,34 +992,57 @@ struct Smem {
 // (g = e / L, k = e % L). Every layout has at least G L threads, so each
 // thread moves at most one element of each field, and all loads of a stage
 // are issued before any store: one memory round trip per stage.
+SHD int div_nx(const MpArgs& A, int64_t n) { return (int)(((uint64_t)(uint32_t)n * A.by_nx.m) >> A.by_nx.s); }
+
 struct StageMap {
   int g, k, gk, kk;
   bool ok, okk;
   int64_t i, j, ik, jk;
   template <int G>
   SHD void set(const MpArgs& A, int tid, int64_t c0) {
-    const int L = A.nz;
     g = tid % G;
     k = tid / G;
     const int64_t col = c0 + g;
-    ok = col < A.ncol && k < L;
-    i = ok ? col % A.nx : 0;
-    j = ok ? col / A.nx : 0;
-    gk = tid / L;
-    kk = tid % L;
+    ok = col < A.ncol && k < A.nz;
+    j = ok ? div_nx(A, col) : 0;
+    i = ok ? col - j * A.nx : 0;
+  }
+  // the k-fastest order
+  template <int G>
+  SHD void set_kfast(const MpArgs& A, int tid, int64_t c0) {
+    gk = tid / A.nz;
+    kk = tid - gk * A.nz;
     const int64_t colk = c0 + gk;
     okk = gk < G && colk < A.ncol;
-    ik = okk ? colk % A.nx : 0;
-    jk = okk ? colk / A.nx : 0;
+    jk = okk ? div_nx(A, colk) : 0;
+    ik = okk ? colk - jk * A.nx : 0;
   }
 };
 
+// With one set of strides in every field of the caller (same_strides: NDSL
+// storages of one shape), the staging forms one offset; otherwise each
+// field its own, in its own memory order. The general form's 64-bit column
+// divisions and 26 address computations were 1,250 of the step's 8,600
+// instructions per warp.
 template <class LY>
 SHD void stage_in(const MpArgs& A, double* sm, int64_t c0) {
   constexpr int RP = LY::RP, G = LY::G;
   StageMap M;
   M.template set<G>(A, threadIdx.x, c0);
   double v[N_IN];
+  if (A.same_strides) {
+    const Fld3& F = A.in[0];
+    const int64_t o = M.i * F.si + M.j * F.sj + (int64_t)M.k * F.sk;
+    const int64_t oq = c0 + M.g + M.k * A.ncol;
+    if (!M.ok) return;
+#pragma unroll
+    for (int f = 0; f < IN_QAZ; ++f) v[f] = A.in[f].p[o];
+    v[IN_QAZ] = A.in[IN_QAZ].p[oq];
+#pragma unroll
+    for (int f = 0; f < N_IN; ++f) sm[(f * G + M.g) * RP + M.k] = v[f];
+    return;
+  }
+  M.template set_kfast<G>(A, threadIdx.x, c0);
 #pragma unroll
   for (int f = 0; f < N_IN; ++f) {
     const Fld3 F = A.in[f];
@@ -1052,9 +1081,31 @@ SHD void stage_out(const MpArgs& A, const double* sm, int64_t c0) {
   const MpConst& K = A.K;
   StageMap M;
   M.template set<G>(A, threadIdx.x, c0);
+  double old[N_OUT];
+  if (A.same_strides) {
+    const Fld3& F = A.in[0];
+    const int64_t o = M.i * F.si + M.j * F.sj + (int64_t)M.k * F.sk;
+    const int64_t oq = c0 + M.g + M.k * A.ncol;
+    if (!M.ok) return;
+    const bool k1 = M.k >= 1;  // the winds' tendencies are written below the top level
+#pragma unroll
+    for (int n = 0; n < OUT_W; ++n) {
+      const int m = out_mode(K, n);
+      old[n] = (m == OM_ADD || (m == OM_ADD_K1 && k1)) ? A.out[n].p[o] : 0.0;
+    }
+#pragma unroll
+    for (int n = 0; n < OUT_W; ++n) {
+      const int m = out_mode(K, n);
+      const double v = sm[(n * G + M.g) * RP + M.k];
+      if (m == OM_SET || m == OM_ADD || (m == OM_ADD_K1 && k1)) A.out[n].p[o] = (m == OM_SET) ? v : old[n] + v;
+    }
+    if (out_mode(K, OUT_W) == OM_SET) A.out[OUT_W].p[o] = sm[(OUT_W * G + M.g) * RP + M.k];
+    A.out[OUT_QAZ].p[oq] = sm[(OUT_QAZ * G + M.g) * RP + M.k];
+    return;
+  }
+  M.template set_kfast<G>(A, threadIdx.x, c0);
   int mode[N_OUT];
   double* dst[N_OUT];
-  double old[N_OUT];
 #pragma unroll
   for (int o = 0; o < N_OUT; ++o) {
     int m = out_mode(K, o);
@@ -1083,9 +1134,22 @@ struct LevState {
   double qv, ql, qr, qi, qs, qg, tz, w;
 };
 struct StepGeom {
-  double dp1, p1, h_var, rh_adj, rh_rain, ccn, c_praut;  // fields_init
+  double dp1, p1;  // fields_init
+  // fields_init's values of the whole column, in shared memory (five doubles
+  // that every level would otherwise keep in registers): written by level 0,
+  // read after the next exchange
+  double* cv;
+  SHD double h_var() const { return cv[0]; }
+  SHD double rh_adj() const { return cv[1]; }
+  SHD double rh_rain() const { return cv[2]; }
+  SHD double ccn() const { return cv[3]; }
+  SHD double c_praut() const { return cv[4]; }
   double den, denfac, dz1, dz;                           // start of each sub-step
 };
+
+// the column's surface totals, after fields_init's five values: kept and read
+// by the bottom level alone
+enum ColumnTotal { CV_RAIN = 5, CV_ICE, CV_SNOW, CV_GRAUPEL };
 
 // fields_init (:27-276) for one level from its input values (defaults on
 // the padding levels k >= L, whose values never reach a real level).
@@ -1118,15 +1182,20 @@ SHD void fields_init(Col& C, const MpConst& K, bool valid, double pt, double qvi
       ccn = qdiv(ccn * K.RDGAS * tzb, p1b);
     }
   }
-  P.ccn = ccn;
-  P.c_praut = K.cpaut * xpowp(ccn * RHOR, -1.0 / 3.0);
+  P.cv = C.cv;
+  const double c_praut = K.cpaut * xpowp(ccn * RHOR, -1.0 / 3.0);
   const double s_leng = qsqrt(qsqrt(area * 1.0e-10));
   const double t_land = K.dw_land * s_leng;
   const double t_ocean = K.dw_ocean * s_leng;
-  double h_var = t_land * land + t_ocean * (1.0 - land);
-  P.h_var = qmin(0.2, qmax(0.01, h_var));
-  P.rh_adj = 1.0 - P.h_var - K.rh_inc;
-  P.rh_rain = qmax(0.35, P.rh_adj - K.rh_inr);
+  const double h_var = qmin(0.2, qmax(0.01, t_land * land + t_ocean * (1.0 - land)));
+  const double rh_adj = 1.0 - h_var - K.rh_inc;
+  if (k == 0) {
+    P.cv[0] = h_var;
+    P.cv[1] = rh_adj;
+    P.cv[2] = qmax(0.35, rh_adj - K.rh_inr);
+    P.cv[3] = ccn;
+    P.cv[4] = c_praut;
+  }
 
   if (K.fix_negative) {
     fix_negative_point(K, S.qv, S.ql, S.qr, S.qi, S.qs, S.qg, S.tz);
@@ -1225,9 +1294,9 @@ SHD void warm_rain(Col& C, const MpConst& K, const MpConstF& KF, bool valid, Lev
     const bool vf = valid && fall;
     if (fall) {
       if constexpr (MIXED)
-        revap_racc_m(K, KF, dt5, P.h_var, qg, qi, ql, qr, qs, qv, tz, P.den, P.denfac);
+        revap_racc_m(K, KF, dt5, P.h_var(), qg, qi, ql, qr, qs, qv, tz, P.den, P.denfac);
       else
-        revap_racc(K, dt5, P.h_var, qg, qi, ql, qr, qs, qv, tz, P.den, P.denfac);
+        revap_racc(K, dt5, P.h_var(), qg, qi, ql, qr, qs, qv, tz, P.den, P.denfac);
     }
     rec.state(0, S);
     const double dm = P.dp1 * (1.0 + qv + ql + qr + qi + qs + qg);
@@ -1237,9 +1306,9 @@ SHD void warm_rain(Col& C, const MpConst& K, const MpConstF& KF, bool valid, Lev
     rec.state(1, S);
     if (fall) {
       if constexpr (MIXED)
-        revap_racc_m(K, KF, dt5, P.h_var, qg, qi, ql, qr, qs, qv, tz, P.den, P.denfac);
+        revap_racc_m(K, KF, dt5, P.h_var(), qg, qi, ql, qr, qs, qv, tz, P.den, P.denfac);
       else
-        revap_racc(K, dt5, P.h_var, qg, qi, ql, qr, qs, qv, tz, P.den, P.denfac);
+        revap_racc(K, dt5, P.h_var(), qg, qi, ql, qr, qs, qv, tz, P.den, P.denfac);
     }
     rec.state(2, S);
   } else {
@@ -1249,22 +1318,22 @@ SHD void warm_rain(Col& C, const MpConst& K, const MpConstF& KF, bool valid, Lev
   }
   if (K.irain_f != 0) {
     if constexpr (MIXED)
-      autoconv_no_subgrid_var_m(K, KF, ql, qr, tz, P.den, P.ccn, P.c_praut);
+      autoconv_no_subgrid_var_m(K, KF, ql, qr, tz, P.den, P.ccn(), P.c_praut());
     else
-      autoconv_no_subgrid_var(K, ql, qr, tz, P.den, P.ccn, P.c_praut);
+      autoconv_no_subgrid_var(K, ql, qr, tz, P.den, P.ccn(), P.c_praut());
   } else {
     double dl;
     if (K.z_slope_liq) {
       dl = mono_slope(C, ql);
       rec.value(0, dl);
-      dl = qmax(dl, qmax(QVMIN, P.h_var * ql));
+      dl = qmax(dl, qmax(QVMIN, P.h_var() * ql));
     } else {
-      dl = qmax(QVMIN, P.h_var * ql);
+      dl = qmax(QVMIN, P.h_var() * ql);
     }
     if constexpr (MIXED)
-      autoconv_subgrid_var_m(K, KF, ql, qr, tz, P.den, P.ccn, P.c_praut, dl);
+      autoconv_subgrid_var_m(K, KF, ql, qr, tz, P.den, P.ccn(), P.c_praut(), dl);
     else
-      autoconv_subgrid_var(K, ql, qr, tz, P.den, P.ccn, P.c_praut, dl);
+      autoconv_subgrid_var(K, ql, qr, tz, P.den, P.ccn(), P.c_praut(), dl);
   }
 }
 
@@ -1272,12 +1341,12 @@ SHD void warm_rain(Col& C, const MpConst& K, const MpConstF& KF, bool valid, Lev
 // implicit falls of ice, snow and graupel with their vertical-velocity
 // transport and heating. Returns the solid flux m1_sol at this level and
 // m1_prev, the one at the level above; the bottom level adds the surface
-// fluxes to ice, snow and graupel. A recorder gets the cloud ice fall speed
+// fluxes to the column's totals. A recorder gets the cloud ice fall speed
 // (value 0).
 template <bool MIXED, class Col, class Rec = NoRec>
 SHD void sedimentation(Col& C, const MpConst& K, const MpConstF& KF, bool valid, LevState& S,
-                       const StepGeom& P, double& vtg, double& vts, double& m1_sol, double& m1_prev, double& ice,
-                       double& snow, double& graupel, unsigned* flags = nullptr, const Rec& rec = Rec()) {
+                       const StepGeom& P, double& vtg, double& vts, double& m1_sol, double& m1_prev,
+                       unsigned* flags = nullptr, const Rec& rec = Rec()) {
   const int k = C.k, L = C.L;
   double &qv = S.qv, &ql = S.ql, &qr = S.qr, &qi = S.qi, &qs = S.qs, &qg = S.qg, &tz = S.tz, &w = S.w;
   const double dp1 = P.dp1, dz = P.dz;
@@ -1344,19 +1413,19 @@ SHD void sedimentation(Col& C, const MpConst& K, const MpConstF& KF, bool valid,
     m1_sol = flux[0];
     m1_prev = fp[0];
     if (K.do_sedi_w) w = w_update(k, w, dm_i, flux[0], vti, fp[0], vp[0]);
-    if (bottom) ice = ice + flux[0];
+    if (bottom) C.cv[CV_ICE] += flux[0];
   }
   if (fs) {
     m1_sol = m1_sol + flux[1];
     m1_prev = m1_prev + fp[1];
     if (K.do_sedi_w) w = w_update(k, w, dm_s, flux[1], vts, fp[1], vp[1]);
-    if (bottom) snow = snow + flux[1];
+    if (bottom) C.cv[CV_SNOW] += flux[1];
   }
   if (fg) {
     m1_sol = m1_sol + flux[2];
     m1_prev = m1_prev + fp[2];
     if (K.do_sedi_w) w = w_update(k, w, dm_g, flux[2], vtg, fp[2], vp[2]);
-    if (bottom) graupel = graupel + flux[2];
+    if (bottom) C.cv[CV_GRAUPEL] += flux[2];
   }
   if (K.do_sedi_heat) sedi_heat(C, K, tz, P.dz1, dp1, qv, ql, qr, qi, qs, qg, m1_sol, m1_prev, valid, K.C_ICE);
 }
@@ -1376,9 +1445,9 @@ SHD void icloud(Col& C, const MpConst& K, const MpConstF& KF, bool valid, LevSta
   if (K.z_slope_ice) {
     di = mono_slope(C, qi);
     rec.value(0, di);
-    di = qmax(di, qmax(QVMIN, P.h_var * qi));
+    di = qmax(di, qmax(QVMIN, P.h_var() * qi));
   } else {
-    di = qmax(QVMIN, P.h_var * qi);
+    di = qmax(QVMIN, P.h_var() * qi);
   }
   if (valid) {
     if constexpr (MIXED)
@@ -1388,10 +1457,10 @@ SHD void icloud(Col& C, const MpConst& K, const MpConstF& KF, bool valid, LevSta
       icloud_processes(K, qg, qi, ql, qr, qs, qv, tz, P.den, P.denfac, vtg, vtr, vts, P.p1, di, q_liq, q_sol, cvm);
     rec.state(0, S);
     if constexpr (MIXED)
-      subgrid_z_proc<double, float>(K, P.h_var, P.rh_adj, P.rh_rain, qa, qg, qi, ql, qr, qs, qv, tz, P.den, P.denfac,
+      subgrid_z_proc<double, float>(K, P.h_var(), P.rh_adj(), P.rh_rain(), qa, qg, qi, ql, qr, qs, qv, tz, P.den, P.denfac,
                                     P.p1, &KF);
     else
-      subgrid_z_proc(K, P.h_var, P.rh_adj, P.rh_rain, qa, qg, qi, ql, qr, qs, qv, tz, P.den, P.denfac, P.p1);
+      subgrid_z_proc(K, P.h_var(), P.rh_adj(), P.rh_rain(), qa, qg, qi, ql, qr, qs, qv, tz, P.den, P.denfac, P.p1);
   }
 }
 
@@ -1422,7 +1491,7 @@ SHD void mp_body(const MpArgs& A, double* sm, double* scr, double* work, const i
   auto TL = [&](int f) -> double& { return tile[(size_t)f * G * RP]; };
 
   const int64_t cc = col < A.ncol ? col : A.ncol - 1;
-  const int64_t ci = cc % A.nx, cj = cc / A.nx;
+  const int64_t cj = div_nx(A, cc), ci = cc - cj * A.nx;
   LevState S;
   StepGeom P;
   double qa = valid ? TL(IN_QAZ) : 0.0;
@@ -1438,7 +1507,10 @@ SHD void mp_body(const MpArgs& A, double* sm, double* scr, double* work, const i
               valid ? TL(IN_DELP) : 1.0, valid ? TL(IN_W) : 0.0, valid ? TL(IN_DELZ) : -100.0,
               A.land.p[ci * A.land.si + cj * A.land.sj], A.area.p[ci * A.area.si + cj * A.area.sj], S, P);
 
-  double rain = 0.0, snow = 0.0, ice = 0.0, graupel = 0.0;
+  if (k == L - 1) {
+#pragma unroll
+    for (int n = CV_RAIN; n <= CV_GRAUPEL; ++n) C.cv[n] = 0.0;
+  }
 #pragma unroll 1
   for (int it = 0; it < K.ntimes; ++it) {
     unsigned fl = 0u;  // this sub-step's column flags (FLAGS only)
@@ -1452,12 +1524,11 @@ SHD void mp_body(const MpArgs& A, double* sm, double* scr, double* work, const i
       bool falls = false;
       warm_rain<MIXED>(C, K, KF, valid, S, P, vtr, m1_rain, mp_rain, FLAGS ? &falls : nullptr);
       if constexpr (FLAGS) fl |= falls ? (is_first ? FLAG_RAIN_FALLS_1 : FLAG_RAIN_FALLS_2) : 0u;
-      if (k == L - 1) rain = rain + m1_rain;
+      if (k == L - 1) C.cv[CV_RAIN] += m1_rain;
       m1 = is_first ? m1 + m1_rain : m1 + m1_rain + m1_sol;
       mp = is_first ? mp + mp_rain : mp + mp_rain + mp_sol;
       if (!is_first) break;
-      sedimentation<MIXED>(C, K, KF, valid, S, P, vtg, vts, m1_sol, mp_sol, ice, snow, graupel,
-                           FLAGS ? &fl : nullptr);
+      sedimentation<MIXED>(C, K, KF, valid, S, P, vtg, vts, m1_sol, mp_sol, FLAGS ? &fl : nullptr);
     }
     icloud<MIXED>(C, K, KF, valid, S, P, qa, vtg, vtr, vts);
     if constexpr (FLAGS) {
@@ -1517,13 +1588,15 @@ SHD void mp_body(const MpArgs& A, double* sm, double* scr, double* work, const i
     TL(OUT_QAZ) = qa;
     // the device error word: the first column (+ 1) that produced a NaN or
     // an infinity, for the host to read after the step (never traps)
-    if (A.err && !(isfinite(inc_pt) && isfinite(inc_qv) && isfinite(inc_ql) && isfinite(inc_qr) &&
-                   isfinite(inc_qi) && isfinite(inc_qs) && isfinite(inc_qg) && isfinite(inc_qa) &&
-                   isfinite(inc_u) && isfinite(inc_v) && isfinite(w) && isfinite(qa)))
-      atomicCAS(A.err, 0, (int)(col + 1));
+    // (x 0 is NaN for an infinity or a NaN, and 0 otherwise)
+    double z = inc_pt * 0.0;
+    for (const double x : {inc_qv, inc_ql, inc_qr, inc_qi, inc_qs, inc_qg, inc_qa, inc_u, inc_v, w, qa})
+      z = __fma_rn(x, 0.0, z);
+    if (A.err && !(z == 0.0)) atomicCAS(A.err, 0, (int)(col + 1));
   }
   if (k == L - 1 && col_ok) {
     const double convt = 86400.0 * K.rdt * K.RGRAV;
+    const double rain = C.cv[CV_RAIN], ice = C.cv[CV_ICE], snow = C.cv[CV_SNOW], graupel = C.cv[CV_GRAUPEL];
     if (A.rain) A.rain[col] = rain * convt;
     if (A.snow) A.snow[col] = snow * convt;
     if (A.ice) A.ice[col] = ice * convt;
@@ -1585,6 +1658,7 @@ SHD void stage_in_async(const MpArgs& A, double* sm, int64_t c0) {
   const MpConst& K = A.K;
   StageMap M;
   M.template set<G>(A, threadIdx.x, c0);
+  M.template set_kfast<G>(A, threadIdx.x, c0);
 #pragma unroll
   for (int r = 0; r < NT; ++r) {
     if (r >= N_IN) {
@@ -1609,6 +1683,7 @@ SHD void stage_out_tiled(const MpArgs& A, const double* sm, int64_t c0) {
   const MpConst& K = A.K;
   StageMap M;
   M.template set<G>(A, threadIdx.x, c0);
+  M.template set_kfast<G>(A, threadIdx.x, c0);
 #pragma unroll
   for (int o = 0; o < N_OUT; ++o) {
     int m = out_mode(K, o);

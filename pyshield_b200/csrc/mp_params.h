@@ -65,6 +65,19 @@ struct Fld2 {
   int64_t si, sj;
 };
 
+// n / d for 0 <= n < 2^31 as a multiply and a shift: with 2^(s - 1) < d <= 2^s
+// and m = ceil(2^(31 + s) / d), the excess n (m d - 2^(31 + s)) stays below
+// 2^(31 + s). (A 64-bit division is about a hundred instructions.)
+struct FastDiv {
+  uint32_t m, s;
+};
+inline FastDiv fast_div(int d) {
+  FastDiv f{0, 31};
+  while ((int64_t(1) << (f.s - 31)) < d) ++f.s;
+  f.m = (uint32_t)(((uint64_t(1) << f.s) + (uint64_t)d - 1) / (uint64_t)d);
+  return f;
+}
+
 // Input tiles staged in shared memory, in this order.
 enum InField {
   IN_PT = 0, IN_QV, IN_QL, IN_QR, IN_QI, IN_QS, IN_QG, IN_QA, IN_UA, IN_VA, IN_DELP, IN_DELZ, IN_W, IN_QAZ,
@@ -81,6 +94,10 @@ struct MpArgs {
   MpConstF KF;
   int nx, ny, nz;
   int64_t ncol;
+  FastDiv by_nx;
+  // the caller's fields all have in[0]'s strides, which are not k-fastest:
+  // one offset serves them (set by plan_layout)
+  int same_strides;
   Fld3 in[N_IN];
   Fld3 out[N_OUT];
   Fld2 land, area;
@@ -90,6 +107,17 @@ struct MpArgs {
   // only by the flag-recording launch; null otherwise
   int* flags;
 };
+
+// The staging's precomputed values, from the domain and the fields' strides.
+inline void plan_layout(MpArgs& A) {
+  A.by_nx = fast_div(A.nx);
+  const Fld3& a = A.in[0];
+  bool same = a.sk != 1;
+  auto like = [&](const Fld3& f) { return f.si == a.si && f.sj == a.sj && f.sk == a.sk; };
+  for (int f = 1; f < IN_QAZ; ++f) same = same && like(A.in[f]);
+  for (int o = 0; o < OUT_QAZ; ++o) same = same && like(A.out[o]);
+  A.same_strides = same ? 1 : 0;
+}
 
 // Bits of the per-column, per-sub-step flags word: which species fall (the
 // reference's column-wide no_fall == 0, microphysics.py:349-368 for rain in

@@ -898,14 +898,13 @@ __global__ void __launch_bounds__(LY::THREADS, MINB) vjp_replay_kernel(const __g
     W.sp(SP_P1)[p] = P.p1;
   }
   if (head) {
-    W.sc(SC_HVAR)[cc] = P.h_var;
-    W.sc(SC_RHADJ)[cc] = P.rh_adj;
-    W.sc(SC_RHRAIN)[cc] = P.rh_rain;
-    W.sc(SC_CCN)[cc] = P.ccn;
-    W.sc(SC_CPRAUT)[cc] = P.c_praut;
+    W.sc(SC_HVAR)[cc] = P.h_var();
+    W.sc(SC_RHADJ)[cc] = P.rh_adj();
+    W.sc(SC_RHRAIN)[cc] = P.rh_rain();
+    W.sc(SC_CCN)[cc] = P.ccn();
+    W.sc(SC_CPRAUT)[cc] = P.c_praut();
   }
-  double m1 = 0.0, m1_sol = 0.0, mp_sol = 0.0, vtr = VF_MIN, vtg = VF_MIN, vts = VF_MIN, qa = 0.0, ice = 0.0,
-         snow = 0.0, graupel = 0.0;
+  double m1 = 0.0, m1_sol = 0.0, mp_sol = 0.0, vtr = VF_MIN, vtg = VF_MIN, vts = VF_MIN, qa = 0.0;
   constexpr int NREC = SM::NREC;
   constexpr int64_t RS = (int64_t)G * RP;  // stride between record tiles
   const double* rec = sm + SM::rec;
@@ -953,7 +952,7 @@ __global__ void __launch_bounds__(LY::THREADS, MINB) vjp_replay_kernel(const __g
       }
       if (pass == 1) break;
       // tiles 0 .. 7: the state after sedimentation; 8, 9, 10: vtg, vts, vti
-      sedimentation<false>(C, K, KF, valid, S, P, vtg, vts, m1_sol, mp_sol, ice, snow, graupel, nullptr,
+      sedimentation<false>(C, K, KF, valid, S, P, vtg, vts, m1_sol, mp_sol, nullptr,
                            VjpRec{nullptr, rt + 10 * RS, nullptr, RS, valid, false, false});
       put_lev(0, S);
       put(8, vtg);
