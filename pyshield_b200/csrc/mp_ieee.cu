@@ -19,6 +19,6 @@
 
 namespace shield {
 
-cudaError_t mp_launch_ieee(const MpArgs& A, cudaStream_t st) { return launch_plain_shapes<false>(A, st); }
+cudaError_t mp_launch_ieee(const MpArgs& A, cudaStream_t st) { return launch_shapes<false, false>(A, st); }
 
 }  // namespace shield

@@ -46,13 +46,20 @@ template <int NW>
 struct Column {
   static constexpr int WP = Tiles<NW>::RP;  // pitch of the work rows
   int w, lane, k, L, bar;
-  static constexpr int CV = 10;  // doubles of the column's own values
+  static constexpr int CV = 10;     // doubles of the column's own values
+  static constexpr int NPARK = 13;  // doubles of a thread's slot (ParkSlot)
   double* scr;   // 2 * SCR doubles
-  double* work;  // 2 * RP doubles, for the sequential vapour borrow
+  double* work;  // 2 * RP doubles, for the sequential vapour borrow: the threads' slots, before they are used
+  double* park;  // this thread's slot
   double* cv;    // CV doubles
   int par;
 
-  SHD void sync() const { asm volatile("bar.sync %0, %1;" ::"r"(bar), "r"(32 * NW) : "memory"); }
+  SHD void sync() const {
+    if (NW == 1)
+      __syncwarp();
+    else
+      asm volatile("bar.sync %0, %1;" ::"r"(bar), "r"(32 * NW) : "memory");
+  }
   SHD double* slot() {
     double* s = scr + par * Tiles<NW>::SCR;
     par ^= 1;
@@ -587,13 +594,16 @@ struct PackedColumn {
   int t, c, k, L, bar;
   int wf;      // first warp of this thread's column
   int off;     // 1: the column starts inside that warp
-  static constexpr int CV = 10;  // doubles of a column's own values
+  static constexpr int CV = 10;     // doubles of a column's own values
+  static constexpr int NPARK = 13;  // doubles of a thread's slot (ParkSlot)
+  static_assert((P + 1) * 2 * WP <= T * NPARK, "the work rows lie in the threads' slots");
   double* scr;   // 2 * SCR doubles
-  double* work;  // this column's two work rows (WP doubles each)
-  double* cv;    // and its CV doubles
+  double* work;  // this column's two work rows (WP doubles each), in the threads' slots before they are used
+  double* park;  // this thread's slot
+  double* cv;    // the column's CV doubles
   int par;
 
-  // scr_grp / work_grp: the group's scratch and its P + 1 columns' work rows and values
+  // scr_grp / work_grp: the group's scratch, and its threads' slots with its P + 1 columns' values
   SHD void init(int t_, int L_, int bar_, double* scr_grp, double* work_grp) {
     t = t_;
     L = L_;
@@ -605,8 +615,9 @@ struct PackedColumn {
     wf = s0 >> 5;
     off = (s0 & 31) != 0;
     scr = scr_grp;
-    work = work_grp + (size_t)c * (2 * WP + CV);
-    cv = work + 2 * WP;
+    work = work_grp + (size_t)c * 2 * WP;
+    park = work_grp + (size_t)t * NPARK;
+    cv = work_grp + (size_t)T * NPARK + c * CV;
     par = 0;
   }
   SHD int w() const { return t >> 5; }
@@ -935,10 +946,11 @@ struct ColumnLayout {
   using Col = Column<NW>;
   static constexpr int G = G_;
   static constexpr int NGRP = G_;
+  static_assert(NW == 1 || G_ <= 15, "barrier ids are 1 + g, of 16 (0 is the block's); a one-warp column uses none");
   static constexpr int THREADS = 32 * NW * G_;
   static constexpr int RP = Tiles<NW>::RP;
   static constexpr int SCR = Tiles<NW>::SCR;
-  static constexpr int WORK = 2 * RP + Col::CV;
+  static constexpr int WORK = THREADS / G_ * Col::NPARK + Col::CV;
   // set up thread tid's column object; returns its block column (G: none)
   static SHD int setup(Col& C, int tid, int L, double* scr, double* work) {
     const int g = tid / (32 * NW);
@@ -949,7 +961,8 @@ struct ColumnLayout {
     C.bar = 1 + g;
     C.scr = scr + (size_t)g * 2 * SCR;
     C.work = work + (size_t)g * WORK;
-    C.cv = C.work + 2 * RP;
+    C.park = C.work + (tid % (32 * NW)) * Col::NPARK;
+    C.cv = C.work + 32 * NW * Col::NPARK;
     C.par = 0;
     return g;
   }
@@ -965,7 +978,7 @@ struct PackedLayout {
   static constexpr int THREADS = 32 * NWG * NGRP_;
   static constexpr int RP = Col::WP;
   static constexpr int SCR = Col::SCR;
-  static constexpr int WORK = (P + 1) * (2 * Col::WP + Col::CV);
+  static constexpr int WORK = 32 * NWG * Col::NPARK + (P + 1) * Col::CV;
   static SHD int setup(Col& C, int tid, int L, double* scr, double* work) {
     const int gi = tid / (32 * NWG);
     C.init(tid % (32 * NWG), L, 1 + gi, scr + (size_t)gi * 2 * SCR, work + (size_t)gi * WORK);
@@ -1133,18 +1146,43 @@ SHD void stage_out(const MpArgs& A, const double* sm, int64_t c0) {
 struct LevState {
   double qv, ql, qr, qi, qs, qg, tz, w;
 };
+// the layer geometry a fall works on (the adjoint's column reverses)
 struct StepGeom {
-  double dp1, p1;  // fields_init
-  // fields_init's values of the whole column, in shared memory (five doubles
-  // that every level would otherwise keep in registers): written by level 0,
-  // read after the next exchange
-  double* cv;
+  double dp1, den, denfac, dz1, dz;
+};
+// What a level keeps between its stages, in shared memory: a slot of N_PARK
+// doubles per thread (an odd count, so that consecutive threads' slots hit
+// distinct banks), and the column's own values. The step is bound by the
+// latency of dependent FP64 work, so resident warps decide its rate (a group
+// takes the same time alone on an SM as with three others: 33 against 42 us
+// at L79), and registers decide those: the state in use stays in registers,
+// these values are read where they are needed.
+enum ParkSlot { PK_W, PK_DP1, PK_P1, PK_DZ, PK_DZ1, PK_DENFAC, PK_M1, PK_MP, PK_M1SOL, PK_MPSOL, PK_VTR, PK_VTG, PK_VTS };
+struct LevelStore {
+  double* pk;  // this thread's slot
+  double* cv;  // the column's values: fields_init's, written by level 0 and read after the next exchange
+  double den;  // density (start of each sub-step)
+  SHD double& w() const { return pk[PK_W]; }      // vertical velocity
+  SHD double& dp1() const { return pk[PK_DP1]; }  // fields_init
+  SHD double& p1() const { return pk[PK_P1]; }
+  SHD double& dz() const { return pk[PK_DZ]; }    // start of each sub-step
+  SHD double& dz1() const { return pk[PK_DZ1]; }
+  SHD double& denfac() const { return pk[PK_DENFAC]; }
+  // the precipitation flux summed over the sub-steps, here and at the level
+  // above; the solid flux of the last sedimentation likewise
+  SHD double& m1() const { return pk[PK_M1]; }
+  SHD double& mp() const { return pk[PK_MP]; }
+  SHD double& m1_sol() const { return pk[PK_M1SOL]; }
+  SHD double& mp_sol() const { return pk[PK_MPSOL]; }
+  // the last fall speeds of rain, graupel and snow
+  SHD double& vtr() const { return pk[PK_VTR]; }
+  SHD double& vtg() const { return pk[PK_VTG]; }
+  SHD double& vts() const { return pk[PK_VTS]; }
   SHD double h_var() const { return cv[0]; }
   SHD double rh_adj() const { return cv[1]; }
   SHD double rh_rain() const { return cv[2]; }
   SHD double ccn() const { return cv[3]; }
   SHD double c_praut() const { return cv[4]; }
-  double den, denfac, dz1, dz;                           // start of each sub-step
 };
 
 // the column's surface totals, after fields_init's five values: kept and read
@@ -1156,21 +1194,21 @@ enum ColumnTotal { CV_RAIN = 5, CV_ICE, CV_SNOW, CV_GRAUPEL };
 template <class Col>
 SHD void fields_init(Col& C, const MpConst& K, bool valid, double pt, double qvi, double qli, double qri,
                      double qii, double qsi, double qgi, double delp, double wz, double dz0, double land, double area,
-                     LevState& S, StepGeom& P) {
+                     LevState& S, LevelStore& P) {
   const int k = C.k, L = C.L;
+  P.pk = C.park;
+  P.cv = C.cv;
   S.tz = pt;
-  P.dp1 = delp;
-  P.dp1 = P.dp1 * (1.0 - qvi);
-  const double omq = qdiv(delp, P.dp1);
+  const double dp1 = delp * (1.0 - qvi);
+  const double omq = qdiv(delp, dp1);
   S.qv = qvi * omq;
   S.ql = qli * omq;
   S.qr = qri * omq;
   S.qi = qii * omq;
   S.qs = qsi * omq;
   S.qg = qgi * omq;
-  const double den0 = qdiv(-P.dp1, K.GRAV * dz0);
-  P.p1 = den0 * K.RDGAS * pt;
-  S.w = wz;
+  const double den0 = qdiv(-dp1, K.GRAV * dz0);
+  const double p1 = den0 * K.RDGAS * pt;
   double ccn;
   if (K.prog_ccn) {
     ccn = 0.0 * 1.0e6;
@@ -1178,11 +1216,10 @@ SHD void fields_init(Col& C, const MpConst& K, bool valid, double pt, double qvi
     ccn = (K.ccn_l * land + K.ccn_o * (1.0 - land)) * 1.0e6;
     if (K.use_ccn) {
       double tzb, p1b;
-      C.bcast2(S.tz, P.p1, L - 1, tzb, p1b);
+      C.bcast2(S.tz, p1, L - 1, tzb, p1b);
       ccn = qdiv(ccn * K.RDGAS * tzb, p1b);
     }
   }
-  P.cv = C.cv;
   const double c_praut = K.cpaut * xpowp(ccn * RHOR, -1.0 / 3.0);
   const double s_leng = qsqrt(qsqrt(area * 1.0e-10));
   const double t_land = K.dw_land * s_leng;
@@ -1208,7 +1245,7 @@ SHD void fields_init(Col& C, const MpConst& K, bool valid, double pt, double qvi
       double* wd = wq + Col::WP;
       if (valid) {
         wq[k] = S.qv;
-        wd[k] = P.dp1;
+        wd[k] = dp1;
       }
       C.sync();
       if (k == 0) {
@@ -1223,37 +1260,46 @@ SHD void fields_init(Col& C, const MpConst& K, bool valid, double pt, double qvi
     if (k < L - 1 && S.qv < 0.0) S.qv = 0.0;
     // bottom layer borrows from the layer above (:253-276): the two levels
     // form the same dq
-    const double x[2] = {S.qv, P.dp1};
+    const double x[2] = {S.qv, dp1};
     double xp[2], xn[2];
     C.template nbrsN<2>(x, xp, xn);
     if (k == L - 2 || k == L - 1) {
       const bool bot = k == L - 1;
-      const double qb = bot ? S.qv : xn[0], db = bot ? P.dp1 : xn[1];
-      const double qb1 = bot ? xp[0] : S.qv, db1 = bot ? xp[1] : P.dp1;
+      const double qb = bot ? S.qv : xn[0], db = bot ? dp1 : xn[1];
+      const double qb1 = bot ? xp[0] : S.qv, db1 = bot ? xp[1] : dp1;
       if ((qb < 0.0) && (qb1 > 0.0)) {
-        const double dq = qdiv(qmin(-qb * db, qb1 * db1), P.dp1);
+        const double dq = qdiv(qmin(-qb * db, qb1 * db1), dp1);
         S.qv = bot ? S.qv + dq : S.qv - dq;
       }
     }
   }
+  // after every read of the borrow's work rows, which these slots overlie
+  // (the exchange above lies between)
+  P.w() = wz;
+  P.dp1() = dp1;
+  P.p1() = p1;
+  P.m1() = 0.0;
+  P.mp() = 0.0;
 }
 
 // density, fall factor and layer thickness at the start of a sub-step
 // (warm_rain with is_first, :349-380)
 template <class Col>
 SHD void substep_geometry(Col& C, const MpConst& K, bool valid, double t0, double dz0, const LevState& S,
-                          StepGeom& P) {
-  const double den0 = qdiv(-P.dp1, K.GRAV * dz0);
-  P.dz1 = qdiv(dz0 * S.tz, t0);
-  P.den = qdiv(den0 * dz0, P.dz1);
-  P.denfac = qsqrt(qdiv(SFCRHO, P.den));
-  P.dz = C.heights(valid ? -P.dz1 : 0.0, K.zs);
+                          LevelStore& P) {
+  const double den0 = qdiv(-P.dp1(), K.GRAV * dz0);
+  const double dz1 = qdiv(dz0 * S.tz, t0);
+  P.den = qdiv(den0 * dz0, dz1);
+  P.dz1() = dz1;
+  P.denfac() = qsqrt(qdiv(SFCRHO, P.den));
+  P.dz() = C.heights(valid ? -dz1 : 0.0, K.zs);
 }
 
 // Recorder of a stage's intermediate states. The forward kernels pass
 // NoRec (every call compiles away); the adjoint's replay passes one that
 // stores the states the reverse sweeps start from.
 struct NoRec {
+  static constexpr bool on = false;
   SHD void state(int, const LevState&) const {}
   SHD void value(int, double) const {}
   SHD void flag(bool) const {}
@@ -1267,10 +1313,11 @@ struct NoRec {
 // fall (1) and after the second evaporation (2), the liquid slope (value 0)
 // and the column's rain-fall decision.
 template <bool MIXED, class Col, class Rec = NoRec>
-SHD void warm_rain(Col& C, const MpConst& K, const MpConstF& KF, bool valid, LevState& S, const StepGeom& P,
-                   double& vtr, double& m1_rain, double& m1_prev, bool* falls = nullptr, const Rec& rec = Rec()) {
+SHD void warm_rain(Col& C, const MpConst& K, const MpConstF& KF, bool valid, LevState& S, const LevelStore& P,
+                   double& m1_rain, double& m1_prev, bool* falls = nullptr, const Rec& rec = Rec()) {
   const int k = C.k;
-  double &qv = S.qv, &ql = S.ql, &qr = S.qr, &qi = S.qi, &qs = S.qs, &qg = S.qg, &tz = S.tz, &w = S.w;
+  double &qv = S.qv, &ql = S.ql, &qr = S.qr, &qi = S.qi, &qs = S.qs, &qg = S.qg, &tz = S.tz;
+  if constexpr (Rec::on) S.w = P.w();
   const double dt5 = 0.5 * K.dt_rain;
   m1_rain = 0.0;
   m1_prev = 0.0;
@@ -1286,7 +1333,8 @@ SHD void warm_rain(Col& C, const MpConst& K, const MpConstF& KF, bool valid, Lev
   C.any_prev(valid && (qr > QRMIN), vt, fall, gfall, vp);
   if (falls) *falls = fall;
   rec.flag(fall);
-  vtr = fall ? vt : VF_MIN;
+  const double vtr = fall ? vt : VF_MIN;
+  P.vtr() = vtr;
   // The fall's vertical operations run whenever a column sharing the
   // barrier has falling rain; a column without it takes part with no mass
   // (valid false), which leaves its state unchanged and its flux zero.
@@ -1294,21 +1342,23 @@ SHD void warm_rain(Col& C, const MpConst& K, const MpConstF& KF, bool valid, Lev
     const bool vf = valid && fall;
     if (fall) {
       if constexpr (MIXED)
-        revap_racc_m(K, KF, dt5, P.h_var(), qg, qi, ql, qr, qs, qv, tz, P.den, P.denfac);
+        revap_racc_m(K, KF, dt5, P.h_var(), qg, qi, ql, qr, qs, qv, tz, P.den, P.denfac());
       else
-        revap_racc(K, dt5, P.h_var(), qg, qi, ql, qr, qs, qv, tz, P.den, P.denfac);
+        revap_racc(K, dt5, P.h_var(), qg, qi, ql, qr, qs, qv, tz, P.den, P.denfac());
     }
     rec.state(0, S);
-    const double dm = P.dp1 * (1.0 + qv + ql + qr + qi + qs + qg);
-    m1_rain = implicit_fall(C, qr, vtr, vp, P.dz, P.dp1, vf, K.dt_rain, m1_prev);
-    if (fall && K.do_sedi_w) w = w_update(k, w, dm, m1_rain, vtr, m1_prev, vp);
-    if (K.do_sedi_heat) sedi_heat(C, K, tz, P.dz1, P.dp1, qv, ql, qr, qi, qs, qg, m1_rain, m1_prev, vf, K.C_LIQ);
+    const double dp1 = P.dp1();
+    const double dm = dp1 * (1.0 + qv + ql + qr + qi + qs + qg);
+    m1_rain = implicit_fall(C, qr, vtr, vp, P.dz(), dp1, vf, K.dt_rain, m1_prev);
+    if (fall && K.do_sedi_w) P.w() = w_update(k, P.w(), dm, m1_rain, vtr, m1_prev, vp);
+    if constexpr (Rec::on) S.w = P.w();
+    if (K.do_sedi_heat) sedi_heat(C, K, tz, P.dz1(), P.dp1(), qv, ql, qr, qi, qs, qg, m1_rain, m1_prev, vf, K.C_LIQ);
     rec.state(1, S);
     if (fall) {
       if constexpr (MIXED)
-        revap_racc_m(K, KF, dt5, P.h_var(), qg, qi, ql, qr, qs, qv, tz, P.den, P.denfac);
+        revap_racc_m(K, KF, dt5, P.h_var(), qg, qi, ql, qr, qs, qv, tz, P.den, P.denfac());
       else
-        revap_racc(K, dt5, P.h_var(), qg, qi, ql, qr, qs, qv, tz, P.den, P.denfac);
+        revap_racc(K, dt5, P.h_var(), qg, qi, ql, qr, qs, qv, tz, P.den, P.denfac());
     }
     rec.state(2, S);
   } else {
@@ -1339,25 +1389,24 @@ SHD void warm_rain(Col& C, const MpConst& K, const MpConstF& KF, bool valid, Lev
 
 // sedimentation (:657-1217): fall speeds, cloud ice melting, and the
 // implicit falls of ice, snow and graupel with their vertical-velocity
-// transport and heating. Returns the solid flux m1_sol at this level and
-// m1_prev, the one at the level above; the bottom level adds the surface
-// fluxes to the column's totals. A recorder gets the cloud ice fall speed
-// (value 0).
+// transport and heating. Stores the solid flux at this level and at the level
+// above; the bottom level adds the surface fluxes to the column's totals. A
+// recorder gets the cloud ice fall speed (value 0).
 template <bool MIXED, class Col, class Rec = NoRec>
 SHD void sedimentation(Col& C, const MpConst& K, const MpConstF& KF, bool valid, LevState& S,
-                       const StepGeom& P, double& vtg, double& vts, double& m1_sol, double& m1_prev,
-                       unsigned* flags = nullptr, const Rec& rec = Rec()) {
+                       const LevelStore& P, unsigned* flags = nullptr, const Rec& rec = Rec()) {
   const int k = C.k, L = C.L;
-  double &qv = S.qv, &ql = S.ql, &qr = S.qr, &qi = S.qi, &qs = S.qs, &qg = S.qg, &tz = S.tz, &w = S.w;
-  const double dp1 = P.dp1, dz = P.dz;
-  double vti;
+  double &qv = S.qv, &ql = S.ql, &qr = S.qr, &qi = S.qi, &qs = S.qs, &qg = S.qg, &tz = S.tz;
+  const double dp1 = P.dp1(), dz = P.dz();
+  double vti, vts, vtg;
   if constexpr (MIXED)
     fall_speed_m(K, KF, qg, qi, qs, tz, P.den, vtg, vti, vts);
   else
     fall_speed(K, qg, qi, qs, tz, P.den, vtg, vti, vts);
   rec.value(0, vti);
-  m1_sol = 0.0;
-  m1_prev = 0.0;
+  P.vtg() = vtg;
+  P.vts() = vts;
+  double m1_sol = 0.0, m1_prev = 0.0;
   // cloud ice melting at and below the first level warmer than tice (:702-746);
   // the fall speeds above come with the same exchange
   const double vt[3] = {vti, vts, vtg};
@@ -1409,6 +1458,7 @@ SHD void sedimentation(Col& C, const MpConst& K, const MpConstF& KF, bool valid,
   const double dm_g = dp1 * (1.0 + qv + ql + qr + qi + qs + qg);
   if (fg && valid) qg = by_dp1(r[2] * dz);
   const bool bottom = k == L - 1;
+  double w = P.w();
   if (fi) {
     m1_sol = flux[0];
     m1_prev = fp[0];
@@ -1427,7 +1477,11 @@ SHD void sedimentation(Col& C, const MpConst& K, const MpConstF& KF, bool valid,
     if (K.do_sedi_w) w = w_update(k, w, dm_g, flux[2], vtg, fp[2], vp[2]);
     if (bottom) C.cv[CV_GRAUPEL] += flux[2];
   }
-  if (K.do_sedi_heat) sedi_heat(C, K, tz, P.dz1, dp1, qv, ql, qr, qi, qs, qg, m1_sol, m1_prev, valid, K.C_ICE);
+  P.w() = w;
+  P.m1_sol() = m1_sol;
+  P.mp_sol() = m1_prev;
+  if constexpr (Rec::on) S.w = w;
+  if (K.do_sedi_heat) sedi_heat(C, K, tz, P.dz1(), dp1, qv, ql, qr, qi, qs, qg, m1_sol, m1_prev, valid, K.C_ICE);
 }
 
 // icloud (:1220-1449): instant melting or freezing, the ice slope, the ice
@@ -1435,8 +1489,8 @@ SHD void sedimentation(Col& C, const MpConst& K, const MpConstF& KF, bool valid,
 // the ice processes and the adjustment (slot 0), the ice slope (value 0) and
 // the cloud ice after melting and freezing (value 1).
 template <bool MIXED, class Col, class Rec = NoRec>
-SHD void icloud(Col& C, const MpConst& K, const MpConstF& KF, bool valid, LevState& S, const StepGeom& P,
-                double& qa, double vtg, double vtr, double vts, const Rec& rec = Rec()) {
+SHD void icloud(Col& C, const MpConst& K, const MpConstF& KF, bool valid, LevState& S, const LevelStore& P,
+                double& qa, const Rec& rec = Rec()) {
   double &qv = S.qv, &ql = S.ql, &qr = S.qr, &qi = S.qi, &qs = S.qs, &qg = S.qg, &tz = S.tz;
   double q_liq, q_sol, cvm;
   icloud_melt_freeze(K, qv, ql, qr, qi, qs, qg, tz, P.den, q_liq, q_sol, cvm);
@@ -1451,16 +1505,17 @@ SHD void icloud(Col& C, const MpConst& K, const MpConstF& KF, bool valid, LevSta
   }
   if (valid) {
     if constexpr (MIXED)
-      icloud_processes_m(K, KF, qg, qi, ql, qr, qs, qv, tz, P.den, P.denfac, vtg, vtr, vts, P.p1, di, q_liq, q_sol,
-                         cvm);
+      icloud_processes_m(K, KF, qg, qi, ql, qr, qs, qv, tz, P.den, P.denfac(), P.vtg(), P.vtr(), P.vts(), P.p1(),
+                         di, q_liq, q_sol, cvm);
     else
-      icloud_processes(K, qg, qi, ql, qr, qs, qv, tz, P.den, P.denfac, vtg, vtr, vts, P.p1, di, q_liq, q_sol, cvm);
+      icloud_processes(K, qg, qi, ql, qr, qs, qv, tz, P.den, P.denfac(), P.vtg(), P.vtr(), P.vts(), P.p1(), di,
+                       q_liq, q_sol, cvm);
     rec.state(0, S);
     if constexpr (MIXED)
-      subgrid_z_proc<double, float>(K, P.h_var(), P.rh_adj(), P.rh_rain(), qa, qg, qi, ql, qr, qs, qv, tz, P.den, P.denfac,
-                                    P.p1, &KF);
+      subgrid_z_proc<double, float>(K, P.h_var(), P.rh_adj(), P.rh_rain(), qa, qg, qi, ql, qr, qs, qv, tz, P.den,
+                                    P.denfac(), P.p1(), &KF);
     else
-      subgrid_z_proc(K, P.h_var(), P.rh_adj(), P.rh_rain(), qa, qg, qi, ql, qr, qs, qv, tz, P.den, P.denfac, P.p1);
+      subgrid_z_proc(K, P.h_var(), P.rh_adj(), P.rh_rain(), qa, qg, qi, ql, qr, qs, qv, tz, P.den, P.denfac(), P.p1());
   }
 }
 
@@ -1493,14 +1548,8 @@ SHD void mp_body(const MpArgs& A, double* sm, double* scr, double* work, const i
   const int64_t cc = col < A.ncol ? col : A.ncol - 1;
   const int64_t cj = div_nx(A, cc), ci = cc - cj * A.nx;
   LevState S;
-  StepGeom P;
-  double qa = valid ? TL(IN_QAZ) : 0.0;
-  // the precipitation flux summed over the sub-steps, here and at the level above
-  double m1 = 0.0, mp = 0.0, m1_sol = 0.0, mp_sol = 0.0, vtr = VF_MIN, vtg = VF_MIN, vts = VF_MIN;
+  LevelStore P;
   P.den = 1.0;
-  P.denfac = 1.0;
-  P.dz1 = -100.0;
-  P.dz = 100.0;
   // ------------------------------------------------ fields_init (:27-276)
   fields_init(C, K, valid, valid ? TL(IN_PT) : 250.0, valid ? TL(IN_QV) : 0.0, valid ? TL(IN_QL) : 0.0,
               valid ? TL(IN_QR) : 0.0, valid ? TL(IN_QI) : 0.0, valid ? TL(IN_QS) : 0.0, valid ? TL(IN_QG) : 0.0,
@@ -1522,21 +1571,21 @@ SHD void mp_body(const MpArgs& A, double* sm, double* scr, double* work, const i
       if (is_first) substep_geometry(C, K, valid, valid ? TL(IN_PT) : 250.0, valid ? TL(IN_DELZ) : -100.0, S, P);
       double m1_rain, mp_rain;
       bool falls = false;
-      warm_rain<MIXED>(C, K, KF, valid, S, P, vtr, m1_rain, mp_rain, FLAGS ? &falls : nullptr);
+      warm_rain<MIXED>(C, K, KF, valid, S, P, m1_rain, mp_rain, FLAGS ? &falls : nullptr);
       if constexpr (FLAGS) fl |= falls ? (is_first ? FLAG_RAIN_FALLS_1 : FLAG_RAIN_FALLS_2) : 0u;
       if (k == L - 1) C.cv[CV_RAIN] += m1_rain;
-      m1 = is_first ? m1 + m1_rain : m1 + m1_rain + m1_sol;
-      mp = is_first ? mp + mp_rain : mp + mp_rain + mp_sol;
+      P.m1() = is_first ? P.m1() + m1_rain : P.m1() + m1_rain + P.m1_sol();
+      P.mp() = is_first ? P.mp() + mp_rain : P.mp() + mp_rain + P.mp_sol();
       if (!is_first) break;
-      sedimentation<MIXED>(C, K, KF, valid, S, P, vtg, vts, m1_sol, mp_sol, FLAGS ? &fl : nullptr);
+      sedimentation<MIXED>(C, K, KF, valid, S, P, FLAGS ? &fl : nullptr);
     }
-    icloud<MIXED>(C, K, KF, valid, S, P, qa, vtg, vtr, vts);
+    icloud<MIXED>(C, K, KF, valid, S, P, TL(IN_QAZ));  // the accumulator stays in its tile
     if constexpr (FLAGS) {
       if (k == 0 && col_ok) A.flags[(int64_t)it * A.ncol + col] = (int)fl;
     }
   }
-  const double qv = S.qv, ql = S.ql, qr = S.qr, qi = S.qi, qs = S.qs, qg = S.qg, tz = S.tz, w = S.w;
-  const double dp1 = P.dp1;
+  const double qv = S.qv, ql = S.ql, qr = S.qr, qi = S.qi, qs = S.qs, qg = S.qg, tz = S.tz;
+  const double dp1 = P.dp1();
   // ------------------------------------------------ fields_update (:1452-1553)
   const double dp0 = valid ? TL(IN_DELP) : 1.0;
   const double u0 = valid ? TL(IN_UA) : 0.0;
@@ -1549,6 +1598,7 @@ SHD void mp_body(const MpArgs& A, double* sm, double* scr, double* work, const i
       av = v0;
       b = 0.0;
     } else {
+      const double mp = P.mp();
       const Divisor<double> by_D(dp0 + mp);
       au = by_D(dp0 * u0);
       av = by_D(dp0 * v0);
@@ -1561,7 +1611,7 @@ SHD void mp_body(const MpArgs& A, double* sm, double* scr, double* work, const i
     const double omq0 = qdiv(dp0, dp1);
     const double qv0 = TL(IN_QV) * omq0, ql0 = TL(IN_QL) * omq0, qr0 = TL(IN_QR) * omq0;
     const double qi0 = TL(IN_QI) * omq0, qs0 = TL(IN_QS) * omq0, qg0 = TL(IN_QG) * omq0;
-    const double t0 = TL(IN_PT), qa0 = TL(IN_QA);
+    const double t0 = TL(IN_PT), qa0 = TL(IN_QA), qa = TL(IN_QAZ), w = P.w();
     const double omq = qdiv(dp1, dp0);
     const double inc_qv = rdt * (qv - qv0) * omq;
     const double inc_ql = rdt * (ql - ql0) * omq;
@@ -1615,116 +1665,6 @@ SHD void mp_block(const MpArgs& A, double* sm, const int64_t c0) {
   mp_body<LY, MIXED, FLAGS>(A, sm, sm + SM::scratch, sm + SM::work, c0);
   __syncthreads();
   stage_out<LY>(A, sm, c0);
-}
-
-// ------------------------------------------------- persistent, double-buffered
-// The same step with the staging taken off the critical path: a persistent
-// block walks its share of the column blocks and, while it computes one,
-// copies the next one's inputs into the other buffer with cp.async: the 14
-// input fields and, where the two buffers have room for them (NT = N_TILE),
-// the 10 old tendencies the step adds to. With NT = N_IN the stage-out reads
-// the old tendencies itself, as the one-block-per-column-block kernel does.
-//
-// Shared memory: two buffers of NT rows per block column, then the scratch
-// and work rows.
-constexpr int N_TILE = N_IN + 10;  // the inputs, then the tendencies read before the update
-
-template <class LY, int NT = N_TILE>
-struct SmemP {
-  static constexpr size_t buf = (size_t)NT * LY::G * LY::RP;
-  static constexpr size_t scratch = 2 * buf;
-  static constexpr size_t work = scratch + (size_t)LY::NGRP * 2 * LY::SCR;
-  static constexpr size_t total = work + (size_t)LY::NGRP * LY::WORK;
-  static constexpr size_t bytes = total * sizeof(double);
-};
-
-SHD void cp_async8(double* dst_smem, const double* src) {
-  const unsigned d = (unsigned)__cvta_generic_to_shared(dst_smem);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d), "l"(src) : "memory");
-}
-SHD void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-SHD void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
-
-// Tile row of the old value of tendency o (o < 10), after the inputs.
-SHD int tend_row(int o) { return N_IN + o; }
-
-SHD const Fld3& tile_src(const MpArgs& A, int r) { return r < N_IN ? A.in[r] : A.out[r - N_IN]; }
-
-// stage_in's mapping, each element copied asynchronously (no register pass):
-// the first NT tile rows (the inputs, then the old tendencies).
-template <class LY, int NT = N_TILE>
-SHD void stage_in_async(const MpArgs& A, double* sm, int64_t c0) {
-  constexpr int RP = LY::RP, G = LY::G;
-  const MpConst& K = A.K;
-  StageMap M;
-  M.template set<G>(A, threadIdx.x, c0);
-  M.template set_kfast<G>(A, threadIdx.x, c0);
-#pragma unroll
-  for (int r = 0; r < NT; ++r) {
-    if (r >= N_IN) {
-      // a tendency the update adds to (stage_out's OM_ADD / OM_ADD_K1 fields)
-      const int o = r - N_IN;
-      if ((o == OUT_UDT || o == OUT_VDT) && !K.sedi_transport) continue;
-      if (o == OUT_QA_DT && K.do_qa) continue;
-    }
-    const Fld3& F = tile_src(A, r);
-    if (F.sk == 1) {
-      if (M.okk) cp_async8(&sm[(r * G + M.gk) * RP + M.kk], F.p + M.ik * F.si + M.jk * F.sj + M.kk);
-    } else if (M.ok) {
-      cp_async8(&sm[(r * G + M.g) * RP + M.k], F.p + M.i * F.si + M.j * F.sj + (int64_t)M.k * F.sk);
-    }
-  }
-}
-
-// stage_out with the old tendencies taken from the tile.
-template <class LY>
-SHD void stage_out_tiled(const MpArgs& A, const double* sm, int64_t c0) {
-  constexpr int RP = LY::RP, G = LY::G;
-  const MpConst& K = A.K;
-  StageMap M;
-  M.template set<G>(A, threadIdx.x, c0);
-  M.template set_kfast<G>(A, threadIdx.x, c0);
-#pragma unroll
-  for (int o = 0; o < N_OUT; ++o) {
-    int m = out_mode(K, o);
-    const Fld3 F = A.out[o];
-    const bool kf = F.sk == 1;
-    const int lev = kf ? M.kk : M.k;
-    if (!(kf ? M.okk : M.ok) || (m == OM_ADD_K1 && lev < 1)) m = OM_SKIP;
-    if (m == OM_SKIP) continue;
-    const int gg = kf ? M.gk : M.g;
-    const double v = sm[(o * G + gg) * RP + lev];
-    double* dst = kf ? F.p + M.ik * F.si + M.jk * F.sj + M.kk : F.p + M.i * F.si + M.j * F.sj + (int64_t)M.k * F.sk;
-    *dst = (m == OM_SET) ? v : sm[(tend_row(o) * G + gg) * RP + lev] + v;
-  }
-}
-
-template <class LY, int MINB, bool MIXED, int NT>
-__global__ void __launch_bounds__(LY::THREADS, MINB)
-    mp_step_persistent_kernel(const __grid_constant__ MpArgs A, const int64_t nblk) {
-  extern __shared__ double sm[];
-  using SP = SmemP<LY, NT>;
-  constexpr int G = LY::G;
-  double* const scr = sm + SP::scratch;
-  double* const work = sm + SP::work;
-  int64_t b = blockIdx.x;
-  if (b < nblk) stage_in_async<LY, NT>(A, sm, b * G);
-  cp_async_commit();
-  for (int it = 0; b < nblk; b += gridDim.x, ++it) {
-    double* const cur = sm + (it & 1) * SP::buf;
-    double* const nxt = sm + ((it + 1) & 1) * SP::buf;
-    cp_async_wait_all();
-    __syncthreads();  // this block's inputs have landed; the previous one's stage-out is done with nxt
-    if (b + gridDim.x < nblk) stage_in_async<LY, NT>(A, nxt, (b + gridDim.x) * G);
-    cp_async_commit();
-    mp_body<LY, MIXED>(A, cur, scr, work, b * G);
-    __syncthreads();
-    if constexpr (NT == N_TILE)
-      stage_out_tiled<LY>(A, cur, b * G);
-    else
-      stage_out<LY>(A, cur, b * G);
-  }
-  cp_async_wait_all();
 }
 
 template <class LY, int MINB, bool MIXED, bool FLAGS = false>
@@ -1787,102 +1727,69 @@ __global__ void __launch_bounds__(LY::THREADS, MINB)
   }
 }
 
-#ifndef SHIELD_PREFETCH_INPUTS_ONLY
-#define SHIELD_PREFETCH_INPUTS_ONLY 0
-#endif
-
-// Launch the step over ceil(ncol / G) column blocks. PERSIST: as many
-// persistent, double-buffered blocks as fit on the device at once, each
-// walking every gridDim.x-th column block; else one block per column block,
-// scheduled by the hardware.
-template <class LY, int MINB, bool MIXED, bool PERSIST, bool FLAGS = false>
+// Launch the step over ceil(ncol / G) column blocks.
+template <class LY, bool MIXED, bool FLAGS = false>
 cudaError_t launch_step(const MpArgs& A, cudaStream_t st) {
   constexpr int G = LY::G;
-  const int64_t nblk = (A.ncol + G - 1) / G;
-  const int threads = LY::THREADS;
-  if (PERSIST) {
-    // the old tendencies join the prefetch where both buffers have room
-    constexpr bool kTend = SmemP<LY, N_TILE>::bytes <= 220 * 1024 && !SHIELD_PREFETCH_INPUTS_ONLY;
-    constexpr int NT = kTend ? N_TILE : N_IN;
-    auto kern = mp_step_persistent_kernel<LY, MINB, MIXED, NT>;
-    const size_t smem = SmemP<LY, NT>::bytes;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    int dev = 0, nsm = 0, per_sm = 0;
-    if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
-    if ((e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
-    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem)) != cudaSuccess) return e;
-    if (per_sm < 1) per_sm = 1;
-    const int64_t resident = (int64_t)nsm * per_sm;
-    const int64_t grid = nblk < resident ? nblk : resident;
-    kern<<<(unsigned)grid, threads, smem, st>>>(A, nblk);
-    return cudaGetLastError();
-  }
-  auto kern = mp_step_kernel<LY, MINB, MIXED, FLAGS>;
+  auto kern = mp_step_kernel<LY, 1, MIXED, FLAGS>;
   const size_t smem = Smem<LY>::bytes;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  kern<<<(unsigned)nblk, threads, smem, st>>>(A);
+  kern<<<(unsigned)((A.ncol + G - 1) / G), LY::THREADS, smem, st>>>(A);
   return cudaGetLastError();
 }
 
-// Launch shape of 65..80 levels (L79): two columns on each group of 5 warps
-// (PackedLayout), SHIELD_PACK_NGRP groups per block, __launch_bounds__
-// minimum SHIELD_PACK_MINB blocks per SM. Every launch of this level range
-// (plain, mixed, flag-recording, ensemble) packs two columns per 5 warps,
-// so a column's arithmetic, and with it its rounding, is the same in all.
-// Measured at C96 L79 (ms per step, plain / mixed; the register cap is
-// 65,536 / threads): 2 groups (320 threads, 168 registers) 5.70 / 4.23,
-// 3 groups (480, 128 with spills) 4.16 / 3.17, 4 groups (640, 96 with spills)
-// 3.65 / 2.50, 5 groups 4.09 / 2.61, 6 groups 3.81 / 2.65; one column per 3
-// warps, 4 columns per block (12 warps, 160 registers) was 5.66 / 3.65. The
-// step is bound by the latency of dependent FP64 work, so resident warps
-// count for more than spilled registers.
-#ifndef SHIELD_PACK_NGRP
-#define SHIELD_PACK_NGRP 4
-#endif
-#ifndef SHIELD_PACK_MINB
-#define SHIELD_PACK_MINB 1
-#endif
-#ifndef SHIELD_PACK_NWG
-#define SHIELD_PACK_NWG 5
-#endif
-#ifndef SHIELD_PACK_P
-#define SHIELD_PACK_P 2
-#endif
-using Packed80 = PackedLayout<SHIELD_PACK_NWG, SHIELD_PACK_P, SHIELD_PACK_NGRP>;
-constexpr int PACK80_MINB = SHIELD_PACK_MINB;
+// The first of the layouts (in the order of their columns per block) whose
+// blocks fit the SMs in one wave, else the last: the step of a group of warps
+// waits on its own FP64 latency, so a domain that leaves SMs idle runs sooner
+// with fewer columns per block (144 columns of L79: 33 us with 2 per block,
+// 35 with 4, 38 with 6, 41 with 8), while a large one wants the block that
+// keeps the SM busiest.
+constexpr int B200_SMS = 148;
+template <bool MIXED, bool FLAGS, class LY, class... More>
+cudaError_t launch_fitting(const MpArgs& A, cudaStream_t st) {
+  if constexpr (sizeof...(More) > 0) {
+    if (A.ncol > (int64_t)LY::G * B200_SMS) return launch_fitting<MIXED, FLAGS, More...>(A, st);
+  }
+  return launch_step<LY, MIXED, FLAGS>(A, st);
+}
+
+// 65..80 levels (L79): two columns on each group of 5 warps (PackedLayout).
+// Every launch of this level range (plain, mixed, flag-recording, ensemble)
+// packs two columns per 5 warps, so a column's arithmetic, and with it its
+// rounding, is the same in all. Groups per block at C96 L79 (ms per step,
+// plain / mixed; the register cap is 65,536 / threads): 3 groups (480
+// threads, 128 registers) 2.26 / 1.76, 4 groups (640, 96) 1.89 / 1.38,
+// 5 groups (800, 72) 1.98 / 1.43, 6 groups (960, 64) 2.24 / 1.58: beyond 4
+// the registers no longer hold the state in use.
 constexpr int PACK80_LMIN = 65, PACK80_LMAX = 80;
+using Packed80 = PackedLayout<5, 2, 4>;
 
-// Launch shape for 81-96 levels: columns per block and the minimum resident
-// blocks per SM given to __launch_bounds__ (which caps the registers per
-// thread). Four columns per block (one 384-thread block per SM) measured
-// fastest: the staging then reads whole 32-byte sectors. 65-80 levels (L79)
-// pack two columns per 5 warps (Packed80).
-#ifndef SHIELD_NW3_G
-#define SHIELD_NW3_G 4
-#endif
-#ifndef SHIELD_NW3_MINB
-#define SHIELD_NW3_MINB 1
-#endif
-// 97..128 levels (L127): columns per block of 4 warps each. C96 L127 (ms):
-// 4 columns (512 threads, 128 registers) 6.29, 5 columns (640, 96) 5.94,
-// 6 columns (768, 80) 5.99.
-#ifndef SHIELD_NW4_G
-#define SHIELD_NW4_G 5
-#endif
-
-// The plain form's launch for each level range (FLAGS: with the column flags
-// recorded).
-template <bool FLAGS>
-cudaError_t launch_plain_shapes(const MpArgs& A, cudaStream_t st) {
+// The launch for each level range. The widest block of a range holds 24 warps
+// (80 registers; six warps per scheduler) where whole columns allow. C96
+// (ms, plain / mixed), by columns per block: L31 8: 0.84 / 0.50, 15: 0.82 /
+// 0.57, 24: 0.70 / 0.50; L63 8: 1.73 / 1.22, 10: 1.62 / 1.13, 12: 1.57 / 1.09,
+// 14: 1.67 / 1.18; L90 4: 2.87 / 2.13, 6: 2.46 / 1.76, 7: 2.36 / 1.68,
+// 8: 2.06 / 1.52, 9: 2.19 / 1.55; L127 4: 3.51 / 2.55, 5: 3.30 / 2.36,
+// 6: 3.22 / 2.27, 7 (28 warps, 72 registers): 3.16 / 2.19, 8: 3.40 / 2.33.
+// At L127 the 7-column block is the faster one only when its waves are many
+// (3,233 columns, 4 waves of either: 0.226 against 0.205).
+template <bool MIXED, bool FLAGS>
+cudaError_t launch_shapes(const MpArgs& A, cudaStream_t st) {
   const int L = A.nz;
-  if (L <= 32) return launch_step<ColumnLayout<1, 4>, 2, false, false, FLAGS>(A, st);
-  if (L <= 64) return launch_step<ColumnLayout<2, 2>, 2, false, false, FLAGS>(A, st);
-  if (L <= PACK80_LMAX) return launch_step<Packed80, PACK80_MINB, false, false, FLAGS>(A, st);
-  if (L <= 96) return launch_step<ColumnLayout<3, SHIELD_NW3_G>, SHIELD_NW3_MINB, false, false, FLAGS>(A, st);
-  if (L <= 128) return launch_step<ColumnLayout<4, SHIELD_NW4_G>, 1, false, false, FLAGS>(A, st);
-  return launch_step<ColumnLayout<8, 1>, 2, false, false, FLAGS>(A, st);
+  if (L <= 32) return launch_fitting<MIXED, FLAGS, ColumnLayout<1, 8>, ColumnLayout<1, 24>>(A, st);
+  if (L <= 64)
+    return launch_fitting<MIXED, FLAGS, ColumnLayout<2, 4>, ColumnLayout<2, 8>, ColumnLayout<2, 12>>(A, st);
+  if (L <= PACK80_LMAX)
+    return launch_fitting<MIXED, FLAGS, PackedLayout<5, 2, 1>, PackedLayout<5, 2, 2>, PackedLayout<5, 2, 3>,
+                          Packed80>(A, st);
+  if (L <= 96)
+    return launch_fitting<MIXED, FLAGS, ColumnLayout<3, 2>, ColumnLayout<3, 4>, ColumnLayout<3, 8>>(A, st);
+  if (L <= 128) {
+    if (A.ncol > 8 * 7 * B200_SMS) return launch_step<ColumnLayout<4, 7>, MIXED, FLAGS>(A, st);
+    return launch_fitting<MIXED, FLAGS, ColumnLayout<4, 2>, ColumnLayout<4, 4>, ColumnLayout<4, 6>>(A, st);
+  }
+  return launch_fitting<MIXED, FLAGS, ColumnLayout<8, 1>, ColumnLayout<8, 3>>(A, st);
 }
 
 // Launch of the ensemble kernel with `grid` persistent blocks; `counter`

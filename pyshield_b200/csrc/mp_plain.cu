@@ -41,10 +41,10 @@ __global__ void gather2d(const double* p, int64_t si, int64_t sj, int nx, int64_
 
 int mp_max_levels() { return 256; }
 
-cudaError_t mp_launch_plain(const MpArgs& A, cudaStream_t st) { return launch_plain_shapes<false>(A, st); }
+cudaError_t mp_launch_plain(const MpArgs& A, cudaStream_t st) { return launch_shapes<false, false>(A, st); }
 
 // The same launches with the column flags recorded (A.flags non-null).
-cudaError_t mp_launch_plain_flags(const MpArgs& A, cudaStream_t st) { return launch_plain_shapes<true>(A, st); }
+cudaError_t mp_launch_plain_flags(const MpArgs& A, cudaStream_t st) { return launch_shapes<false, true>(A, st); }
 
 cudaError_t mp_launch_mixed(const MpArgs& A, cudaStream_t st);
 
@@ -80,12 +80,12 @@ cudaError_t mp_launch_ensemble_plain(const MpArgs* members, const int64_t* offs,
     if (G == 6) return launch_ensemble<PackedLayout<5, 2, 3>, 1, false>(members, offs, nm, counter, grid, st);
     if (G == 8) return launch_ensemble<PackedLayout<5, 2, 4>, 1, false>(members, offs, nm, counter, grid, st);
   } else if (nz <= 96) {
-    if (G == 1) return launch_ensemble<ColumnLayout<3, 1>, 4, false>(members, offs, nm, counter, grid, st);
-    if (G == 2) return launch_ensemble<ColumnLayout<3, 2>, 2, false>(members, offs, nm, counter, grid, st);
-    if (G == 4) return launch_ensemble<ColumnLayout<3, 4>, 1, false>(members, offs, nm, counter, grid, st);
+    if (G == 1) return launch_ensemble<ColumnLayout<3, 1>, 8, false>(members, offs, nm, counter, grid, st);
+    if (G == 2) return launch_ensemble<ColumnLayout<3, 2>, 4, false>(members, offs, nm, counter, grid, st);
+    if (G == 4) return launch_ensemble<ColumnLayout<3, 4>, 2, false>(members, offs, nm, counter, grid, st);
   } else if (nz <= 128) {
-    if (G == 1) return launch_ensemble<ColumnLayout<4, 1>, 4, false>(members, offs, nm, counter, grid, st);
-    if (G == 2) return launch_ensemble<ColumnLayout<4, 2>, 2, false>(members, offs, nm, counter, grid, st);
+    if (G == 1) return launch_ensemble<ColumnLayout<4, 1>, 6, false>(members, offs, nm, counter, grid, st);
+    if (G == 2) return launch_ensemble<ColumnLayout<4, 2>, 3, false>(members, offs, nm, counter, grid, st);
     if (G == 4) return launch_ensemble<ColumnLayout<4, 4>, 1, false>(members, offs, nm, counter, grid, st);
   }
   return cudaErrorInvalidValue;

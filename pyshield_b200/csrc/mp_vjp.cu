@@ -172,6 +172,7 @@ SHD void store_lev(double* q, int64_t npts, const LevState& S) {
 // A warm_rain recorder (full false) stores the fields its stage changed
 // into the pass's block at `st`; icloud's (full true) the whole state.
 struct VjpRec {
+  static constexpr bool on = true;
   double *st, *val, *flg;
   int64_t npts;
   bool valid, head, full;
@@ -886,16 +887,13 @@ __global__ void __launch_bounds__(LY::THREADS, MINB) vjp_replay_kernel(const __g
   const double area = A.area.p[ci * A.area.si + cj * A.area.sj];
   const double pt = TI(IN_PT, 250.0), dz0 = TI(IN_DELZ, -100.0);
   LevState S;
-  StepGeom P;
+  LevelStore P;
   P.den = 1.0;
-  P.denfac = 1.0;
-  P.dz1 = -100.0;
-  P.dz = 100.0;
   fields_init(C, K, valid, pt, TI(IN_QV, 0.0), TI(IN_QL, 0.0), TI(IN_QR, 0.0), TI(IN_QI, 0.0), TI(IN_QS, 0.0),
               TI(IN_QG, 0.0), TI(IN_DELP, 1.0), TI(IN_W, 0.0), dz0, land, area, S, P);
   if (valid) {
-    W.sp(SP_DP1)[p] = P.dp1;
-    W.sp(SP_P1)[p] = P.p1;
+    W.sp(SP_DP1)[p] = P.dp1();
+    W.sp(SP_P1)[p] = P.p1();
   }
   if (head) {
     W.sc(SC_HVAR)[cc] = P.h_var();
@@ -904,7 +902,7 @@ __global__ void __launch_bounds__(LY::THREADS, MINB) vjp_replay_kernel(const __g
     W.sc(SC_CCN)[cc] = P.ccn();
     W.sc(SC_CPRAUT)[cc] = P.c_praut();
   }
-  double m1 = 0.0, m1_sol = 0.0, mp_sol = 0.0, vtr = VF_MIN, vtg = VF_MIN, vts = VF_MIN, qa = 0.0;
+  double m1 = 0.0, qa = 0.0;
   constexpr int NREC = SM::NREC;
   constexpr int64_t RS = (int64_t)G * RP;  // stride between record tiles
   const double* rec = sm + SM::rec;
@@ -919,11 +917,12 @@ __global__ void __launch_bounds__(LY::THREADS, MINB) vjp_replay_kernel(const __g
 #pragma unroll 1
   for (int it = 0; it < nt; ++it) {
     substep_geometry(C, K, valid, pt, dz0, S, P);
+    S.w = P.w();
     put_lev(0, S);
     put(8, P.den);
-    put(9, P.denfac);
-    put(10, P.dz);
-    put(11, P.dz1);
+    put(9, P.denfac());
+    put(10, P.dz());
+    put(11, P.dz1());
     {
       double* d[NREC] = {};
       for (int f = 0; f < 8; ++f) d[f] = W.ckf(it, CKF_E0 + f);
@@ -936,11 +935,11 @@ __global__ void __launch_bounds__(LY::THREADS, MINB) vjp_replay_kernel(const __g
     for (int pass = 0; pass < 2; ++pass) {
       double m1r, mpr;
       // tiles 0 .. 12: the pass's block; 13: the fall speed; 14: the slope
-      warm_rain<false>(C, K, KF, valid, S, P, vtr, m1r, mpr, nullptr,
+      warm_rain<false>(C, K, KF, valid, S, P, m1r, mpr, nullptr,
                        VjpRec{rt, rt + 14 * RS, W.scc(it, pass ? SCC_FALL_B : SCC_FALL_A) + cc, RS, valid, head,
                               false});
-      m1 = (pass == 0) ? m1 + m1r : m1 + m1r + m1_sol;
-      put(13, vtr);
+      m1 = (pass == 0) ? m1 + m1r : m1 + m1r + P.m1_sol();
+      put(13, P.vtr());
       put(11, S.ql);  // autoconversion changed ql and qr
       put(12, S.qr);
       {
@@ -952,11 +951,11 @@ __global__ void __launch_bounds__(LY::THREADS, MINB) vjp_replay_kernel(const __g
       }
       if (pass == 1) break;
       // tiles 0 .. 7: the state after sedimentation; 8, 9, 10: vtg, vts, vti
-      sedimentation<false>(C, K, KF, valid, S, P, vtg, vts, m1_sol, mp_sol, nullptr,
+      sedimentation<false>(C, K, KF, valid, S, P, nullptr,
                            VjpRec{nullptr, rt + 10 * RS, nullptr, RS, valid, false, false});
       put_lev(0, S);
-      put(8, vtg);
-      put(9, vts);
+      put(8, P.vtg());
+      put(9, P.vts());
       {
         double* d[NREC] = {};
         for (int f = 0; f < 8; ++f) d[f] = W.ckf(it, CKF_PASS + f);
@@ -966,7 +965,7 @@ __global__ void __launch_bounds__(LY::THREADS, MINB) vjp_replay_kernel(const __g
     }
     // tiles 0 .. 7: the state before the adjustment; 8, 9: the ice slope and
     // the melted / frozen cloud ice
-    icloud<false>(C, K, KF, valid, S, P, qa, vtg, vtr, vts, VjpRec{rt, rt + 8 * RS, nullptr, RS, valid, false, true});
+    icloud<false>(C, K, KF, valid, S, P, qa, VjpRec{rt, rt + 8 * RS, nullptr, RS, valid, false, true});
     {
       double* d[NREC] = {};
       for (int f = 0; f < 8; ++f) d[f] = W.ckf(it, CKF_E4 + f);
@@ -1848,16 +1847,18 @@ cudaError_t launch_vjp(const VjpArgs& A, cudaStream_t st) {
 
 }  // namespace
 
-// The replay takes the plain step's launch shape for each level range
-// (mp_plain.cu), so that it repeats the step's arithmetic exactly.
+// The replay takes the plain step's packing for each level range, so that it
+// repeats the step's arithmetic exactly; the number of groups in a block is
+// its own (its record tiles fill the shared memory).
+using PackedReplay = PackedLayout<5, 2, 4>;
 cudaError_t mp_launch_vjp(const VjpArgs& A, cudaStream_t st) {
   const int L = A.nz;
-  if (L <= 32) return launch_vjp<ColumnLayout<1, 4>, 2, 1, 2>(A, st);
-  if (L <= 64) return launch_vjp<ColumnLayout<2, 2>, 2, 2, 2>(A, st);
-  if (L <= PACK80_LMAX) return launch_vjp<Packed80, PACK80_MINB, 3, 4>(A, st);
-  if (L <= 96) return launch_vjp<ColumnLayout<3, 4>, 1, 3, 4>(A, st);
+  if (L <= 32) return launch_vjp<ColumnLayout<1, 15>, 1, 1, 2>(A, st);
+  if (L <= 64) return launch_vjp<ColumnLayout<2, 8>, 1, 2, 2>(A, st);
+  if (L <= PACK80_LMAX) return launch_vjp<PackedReplay, 1, 3, 4>(A, st);
+  if (L <= 96) return launch_vjp<ColumnLayout<3, 6>, 1, 3, 4>(A, st);
   if (L <= 128) return launch_vjp<ColumnLayout<4, 5>, 1, 4, 3>(A, st);
-  return launch_vjp<ColumnLayout<8, 1>, 2, 8, 1>(A, st);
+  return launch_vjp<ColumnLayout<8, 2>, 1, 8, 1>(A, st);
 }
 
 }  // namespace shield

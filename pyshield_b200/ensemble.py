@@ -26,7 +26,7 @@ _PRECISION = {"plain": SHIELD_MP_PLAIN, "fp64": SHIELD_MP_PLAIN, "mixed": SHIELD
 # (columns per block, blocks per SM) launch shapes the autotuner times, by
 # level count: 65..80 levels pack two columns per group of 5 warps, so a
 # block holds 2, 4, 6 or 8 columns (shield_mp_ensemble_step)
-CANDIDATES = ((1, 4), (1, 5), (2, 2), (2, 3), (4, 1), (4, 2))
+CANDIDATES = ((1, 6), (1, 8), (2, 3), (2, 4), (4, 1), (4, 2))
 CANDIDATES_PACKED = ((2, 4), (2, 5), (4, 2), (6, 1), (8, 1), (8, 2))
 
 
