@@ -101,121 +101,134 @@ struct AtmArgs {
 };
 
 // The column stencils of UpdateAtmosphereState in one kernel. A block owns
-// a tile of AT_TC = 32 consecutive columns of the full domain (lane =
-// column: every level's accesses are coalesced in the i-fastest layout) and
-// AT_NW warps that share its levels. The pointwise work runs
-// level-parallel; the level-by-level recurrences run in one warp over
-// shared-memory columns, in the reference's order:
+// AT_TC = 32 consecutive columns of the full domain (lane = column: every
+// level's accesses are coalesced in the i-fastest layout) and has AT_LW warps
+// share their levels. The pointwise work runs level-parallel; the
+// level-by-level recurrences run in one warp over shared-memory columns, in
+// the reference's order:
 //   1 (all warps)  the vapour and delp of every level into shared memory;
-//   2 (one warp)   fill_gfs_delp's three sweeps;
+//   2 (one warp)   fill_gfs_delp's three sweeps, where some column of the
+//                  block has a level they change;
 //   3 (all warps)  the filled vapour back (full domain); on the compute
 //                  domain prepare_tendencies_and_update_tracers and moist_cv
 //                  level by level (moist_cv reads what prepare wrote at the
 //                  same level); the new delp into shared memory;
 //   4 (one warp)   update_pressure_and_surface_winds' pe sum;
 //   5 (all warps)  pe, peln, pk.
-// Four warps per block and 49 KB of shared memory let three or four blocks
-// share an SM, so one block's loads overlap another's one-warp recurrences.
-constexpr int AT_TC = 32;
-constexpr int AT_NW = 4;
+// SAME: every field has one set of strides (NDSL storages of one shape), so
+// a level has one offset instead of 29.
+//
+// Bound by memory latency and short rows (256 B of a field and level at a
+// time): 1.39 GB at C96 L79, 0.212 ms at the measured copy rate. Shapes
+// (columns x level warps, blocks per SM; ms at C96 L79 / C96 L127 / 37 x 41
+// L79): 32 x 4, 3 blocks, a general offset per field 0.397 / 0.755 / 0.066;
+// one offset and 32 x 4, 4 blocks 0.388 / 0.704 / 0.070; 32 x 8, 4 blocks
+// 0.347 / 0.578 / 0.049; 32 x 16, 2 blocks 0.327 / 0.546 / 0.039; 64 x 8,
+// 2 blocks 0.324 / 0.642 / 0.054; 128 x 8, one block 0.370. More warps give
+// each phase more loads in flight; beyond 32 a SM the registers spill (48
+// warps 0.406). Without phases 4 and 5 the launch takes 0.288.
+constexpr int AT_TC = 32, AT_LW = 16, AT_MINB = 2;
 
-template <int NKMAX>
-struct AtmSmem {
-  double q[NKMAX][AT_TC];   // the vapour fill_gfs_delp works on
-  double dp[NKMAX][AT_TC];  // the dycore delp it reads; then prepare's new
-                            // delp (each level's thread replaces its own);
-                            // then the interface pressure
-};
-
-template <int NKMAX>
-__global__ void __launch_bounds__(AT_TC * AT_NW) update_atmos_state_kernel(const __grid_constant__ AtmArgs A) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  AtmSmem<NKMAX>& S = *reinterpret_cast<AtmSmem<NKMAX>*>(smem_raw);
-  const int nxf = A.nx + 2 * A.hx, nyf = A.ny + 2 * A.hx;
-  const int64_t ncf = (int64_t)nxf * nyf;
+template <bool SAME>
+__global__ void __launch_bounds__(AT_TC * AT_LW, AT_MINB) update_atmos_state_kernel(const __grid_constant__ AtmArgs A) {
+  // rows of AT_TC columns: the vapour fill_gfs_delp works on, then the dycore
+  // delp it reads; later prepare's new delp (each level's thread replaces
+  // its own), then the interface pressure
+  extern __shared__ double smem[];
   const int nk = A.nz + 1;  // the reference builds these stencils on nz + 1 levels
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int64_t c = (int64_t)blockIdx.x * AT_TC + lane;
+  const int cx = threadIdx.x % AT_TC, w = threadIdx.x / AT_TC;
+  double* const sq = smem + cx;
+  double* const sd = smem + (size_t)nk * AT_TC + cx;
+  const int nxf = A.nx + 2 * A.hx;
+  const int ncf = nxf * (A.ny + 2 * A.hx);
+  const int c = blockIdx.x * AT_TC + cx;
   const bool live = c < ncf;
-  const int64_t i = live ? c % nxf - A.hx : 0, j = live ? c / nxf - A.hx : 0;
+  const int i = live ? c % nxf - A.hx : 0, j = live ? c / nxf - A.hx : 0;
   const bool compute = live && i >= 0 && j >= 0 && i < A.nx && j < A.ny;
   const bool dycore_only = (A.mode & SHIELD_UAS_DYCORE_ONLY) != 0;
   const bool apply = (A.mode & SHIELD_UAS_APPLY) != 0;
   const F3* f = A.f;
+  const int64_t o0 = i * f[0].si + j * f[0].sj, ok = f[0].sk;
+  auto at = [&](const F3& F, int k) -> double& { return SAME ? F.p[o0 + k * ok] : F.at(i, j, k); };
   const F3& Q = dycore_only ? f[D_QV] : f[PU_QV];
   const F3& DP = f[D_DELP];
+  const double q_min = 1.0e-9;
 
   // ---- 1: fill_gfs_delp's inputs, levels 0 .. nk - 2
-  for (int k = w; k < nk - 1; k += AT_NW) {
-    if (live) {
-      S.q[k][lane] = Q.at(i, j, k);
-      S.dp[k][lane] = DP.at(i, j, k);
+  bool fill = false;  // a level that the sweeps would change
+  if (live) {
+#pragma unroll 4
+    for (int k = w; k < nk - 1; k += AT_LW) {
+      const double q = at(Q, k), dp = at(DP, k);
+      sq[k * AT_TC] = q;
+      sd[k * AT_TC] = dp;
+      fill = fill || (k > 0 ? q < q_min : q < 0.0);
     }
   }
-  __syncthreads();
   // ---- 2: fill_gfs_delp(delp, q, 1e-9) (update_atmos_state.py:21-37)
-  if (w == 0 && live) {
-    const double q_min = 1.0e-9;
-    // BACKWARD interval(0, -2): borrow from the (updated) level below
-    double qn = S.q[nk - 2][lane];
-    double dpn = S.dp[nk - 2][lane];
-    for (int k = nk - 3; k >= 0; --k) {
-      double qk = S.q[k][lane];
-      const double dpk = S.dp[k][lane];
-      if (qn < q_min) qk = qk + (qn - q_min) * dpn / dpk;
-      S.q[k][lane] = qk;
-      qn = qk;
-      dpn = dpk;
+  if (__syncthreads_or(fill)) {
+    if (w == 0 && live) {
+      // BACKWARD interval(0, -2): borrow from the (updated) level below
+      double qn = sq[(nk - 2) * AT_TC];
+      double dpn = sd[(nk - 2) * AT_TC];
+      for (int k = nk - 3; k >= 0; --k) {
+        double qk = sq[k * AT_TC];
+        const double dpk = sd[k * AT_TC];
+        if (qn < q_min) qk = qk + (qn - q_min) * dpn / dpk;
+        sq[k * AT_TC] = qk;
+        qn = qk;
+        dpn = dpk;
+      }
+      // PARALLEL interval(1, -1) clamp, FORWARD interval(1, -1) borrow, FORWARD
+      // interval(0, -1) zero: the borrow chain runs on the unzeroed values
+      double qprev = sq[0];
+      double dprev = sd[0];
+      if (qprev < 0.0) sq[0] = 0.0;
+      for (int k = 1; k < nk - 1; ++k) {
+        double qk = sq[k * AT_TC];
+        const double dpk = sd[k * AT_TC];
+        if (qk < q_min) qk = q_min;
+        if (qprev < 0.0) qk = qk + qprev * (dprev) / (dpk);
+        qprev = qk;
+        dprev = dpk;
+        sq[k * AT_TC] = (qk < 0.0) ? 0.0 : qk;
+      }
     }
-    // PARALLEL interval(1, -1) clamp, FORWARD interval(1, -1) borrow, FORWARD
-    // interval(0, -1) zero: the borrow chain runs on the unzeroed values
-    double qprev = S.q[0][lane];
-    double dprev = S.dp[0][lane];
-    if (qprev < 0.0) S.q[0][lane] = 0.0;
-    for (int k = 1; k < nk - 1; ++k) {
-      double qk = S.q[k][lane];
-      const double dpk = S.dp[k][lane];
-      if (qk < q_min) qk = q_min;
-      if (qprev < 0.0) qk = qk + qprev * (dprev) / (dpk);
-      qprev = qk;
-      dprev = dpk;
-      S.q[k][lane] = (qk < 0.0) ? 0.0 : qk;
-    }
+    __syncthreads();
   }
-  __syncthreads();
   // ---- 3: the filled vapour; prepare_tendencies_and_update_tracers and moist_cv.
   // Every load of a level comes before its first store: the fields are
   // separate storages, but the compiler cannot know that, and a store
   // between two loads would make each group of loads wait for the last.
-  for (int k = w; k < nk; k += AT_NW) {
+  for (int k = w; k < nk; k += AT_LW) {
     const bool filled = live && k < nk - 1;
     if (dycore_only || !compute) {
-      if (filled) Q.at(i, j, k) = S.q[k][lane];
+      if (filled) at(Q, k) = sq[k * AT_TC];
       continue;
     }
     const bool prep = k < nk - 1;
     // loads
     double dq[6];
-    dq[0] = f[D_QV].at(i, j, k);
-    dq[1] = f[D_QL].at(i, j, k);
-    dq[2] = f[D_QR].at(i, j, k);
-    dq[3] = f[D_QS].at(i, j, k);
-    dq[4] = f[D_QI].at(i, j, k);
-    dq[5] = f[D_QG].at(i, j, k);
-    double pt_dt = f[PT_DT].at(i, j, k);
-    const double pt = apply ? f[D_PT].at(i, j, k) : 0.0;
+    dq[0] = at(f[D_QV], k);
+    dq[1] = at(f[D_QL], k);
+    dq[2] = at(f[D_QR], k);
+    dq[3] = at(f[D_QS], k);
+    dq[4] = at(f[D_QI], k);
+    dq[5] = at(f[D_QG], k);
+    double pt_dt = at(f[PT_DT], k);
+    const double pt = apply ? at(f[D_PT], k) : 0.0;
     double u_dt = 0.0, v_dt = 0.0, pq[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0}, dp = 0.0;
     if (prep) {
-      u_dt = f[U_DT].at(i, j, k) + (f[U_T1].at(i, j, k) - f[U_T0].at(i, j, k)) * A.rdt;
-      v_dt = f[V_DT].at(i, j, k) + (f[V_T1].at(i, j, k) - f[V_T0].at(i, j, k)) * A.rdt;
-      pt_dt = pt_dt + (f[PU_PT].at(i, j, k) - f[PT_T0].at(i, j, k)) * A.rdt;
-      dp = f[PRSI].at(i, j, k + 1) - f[PRSI].at(i, j, k);
-      pq[0] = S.q[k][lane];
-      pq[1] = f[PU_QL].at(i, j, k);
-      pq[2] = f[PU_QR].at(i, j, k);
-      pq[3] = f[PU_QS].at(i, j, k);
-      pq[4] = f[PU_QI].at(i, j, k);
-      pq[5] = f[PU_QG].at(i, j, k);
+      u_dt = at(f[U_DT], k) + (at(f[U_T1], k) - at(f[U_T0], k)) * A.rdt;
+      v_dt = at(f[V_DT], k) + (at(f[V_T1], k) - at(f[V_T0], k)) * A.rdt;
+      pt_dt = pt_dt + (at(f[PU_PT], k) - at(f[PT_T0], k)) * A.rdt;
+      dp = at(f[PRSI], k + 1) - at(f[PRSI], k);
+      pq[0] = sq[k * AT_TC];
+      pq[1] = at(f[PU_QL], k);
+      pq[2] = at(f[PU_QR], k);
+      pq[3] = at(f[PU_QS], k);
+      pq[4] = at(f[PU_QI], k);
+      pq[5] = at(f[PU_QG], k);
     }
     // prepare_tendencies_and_update_tracers, interval(0, -1)
     double q0 = 0.0;
@@ -224,7 +237,7 @@ __global__ void __launch_bounds__(AT_TC * AT_NW) update_atmos_state_kernel(const
       for (int t = 0; t < 6; ++t) qw[t] = dp * pq[t];
       const double qt = qw[0] + qw[1] + qw[2] + qw[3] + qw[4] + qw[5];
       const double q_sum = dq[0] + dq[1] + dq[2] + dq[3] + dq[4] + dq[5];
-      q0 = S.dp[k][lane] * (1.0 - q_sum) + qt;  // the old delp, read before the store below
+      q0 = sd[k * AT_TC] * (1.0 - q_sum) + qt;  // the old delp, read before the store below
       for (int t = 0; t < 6; ++t) dq[t] = qw[t] / q0;
     }
     // moist_cv(dycore q..., dycore pt, t_dt = pt_dt, CP_AIR, dt), nz + 1 levels
@@ -238,62 +251,64 @@ __global__ void __launch_bounds__(AT_TC * AT_NW) update_atmos_state_kernel(const
       pt_new = pt + pt_dt * A.dt * A.cp_air / cvm;
     }
     // stores
-    if (filled) Q.at(i, j, k) = S.q[k][lane];
+    if (filled) at(Q, k) = sq[k * AT_TC];
     if (prep) {
-      f[U_DT].at(i, j, k) = u_dt;
-      f[V_DT].at(i, j, k) = v_dt;
-      f[D_DELP].at(i, j, k) = q0;
-      S.dp[k][lane] = q0;
-      f[D_QV].at(i, j, k) = dq[0];
-      f[D_QL].at(i, j, k) = dq[1];
-      f[D_QR].at(i, j, k) = dq[2];
-      f[D_QS].at(i, j, k) = dq[3];
-      f[D_QI].at(i, j, k) = dq[4];
-      f[D_QG].at(i, j, k) = dq[5];
+      at(f[U_DT], k) = u_dt;
+      at(f[V_DT], k) = v_dt;
+      at(f[D_DELP], k) = q0;
+      sd[k * AT_TC] = q0;
+      at(f[D_QV], k) = dq[0];
+      at(f[D_QL], k) = dq[1];
+      at(f[D_QR], k) = dq[2];
+      at(f[D_QS], k) = dq[3];
+      at(f[D_QI], k) = dq[4];
+      at(f[D_QG], k) = dq[5];
     }
     if (apply) {
-      f[D_PT].at(i, j, k) = pt_new;
-      f[PT_DT].at(i, j, k) = 0.0;
+      at(f[D_PT], k) = pt_new;
+      at(f[PT_DT], k) = 0.0;
     } else if (prep) {
-      f[PT_DT].at(i, j, k) = pt_dt;
+      at(f[PT_DT], k) = pt_dt;
     }
   }
   if (dycore_only || !apply) return;  // block-uniform: the mode is the launch's
   __syncthreads();
   // ---- 4: update_pressure_and_surface_winds' sum, pe[k] = pe[k - 1] + delp[k - 1]
   if (w == 0 && compute) {
-    double pe = f[PE].at(i, j, 0);
-    double dprev = S.dp[0][lane];
+    double pe = at(f[PE], 0);
+    double dprev = sd[0];
+#pragma unroll 8
     for (int k = 1; k < nk; ++k) {
       pe = pe + dprev;
-      dprev = k < nk - 1 ? S.dp[k][lane] : 0.0;
-      S.dp[k][lane] = pe;
+      dprev = k < nk - 1 ? sd[k * AT_TC] : 0.0;
+      sd[k * AT_TC] = pe;
     }
   }
   __syncthreads();
   // ---- 5: pe, peln, pk on levels 1 .. nk - 1; ps and the surface winds
-  for (int k = 1 + w; k < nk; k += AT_NW) {
+  for (int k = 1 + w; k < nk; k += AT_LW) {
     if (!compute) continue;
-    const double pe = S.dp[k][lane];
-    f[PE].at(i, j, k) = pe;
+    const double pe = sd[k * AT_TC];
+    at(f[PE], k) = pe;
     const double peln = log(pe);
-    f[PELN].at(i, j, k) = peln;
-    f[PK].at(i, j, k) = exp(A.kappa * peln);
+    at(f[PELN], k) = peln;
+    at(f[PK], k) = exp(A.kappa * peln);
   }
   if (w == 0 && compute) {
-    A.ps.at(i, j, 0) = S.dp[nk - 1][lane];
-    A.us.at(i, j, 0) = f[D_UA].at(i, j, nk - 2);
-    A.vs.at(i, j, 0) = f[D_VA].at(i, j, nk - 2);
+    A.ps.at(i, j, 0) = sd[(nk - 1) * AT_TC];
+    A.us.at(i, j, 0) = at(f[D_UA], nk - 2);
+    A.vs.at(i, j, 0) = at(f[D_VA], nk - 2);
   }
 }
 
-template <int NKMAX>
-cudaError_t launch_atmos(const AtmArgs& A, int64_t ncf, cudaStream_t st) {
-  const size_t smem = sizeof(AtmSmem<NKMAX>);
-  auto kern = update_atmos_state_kernel<NKMAX>;
+cudaError_t launch_atmos(const AtmArgs& A, int ncf, cudaStream_t st) {
+  bool same = true;
+  for (const F3& F : A.f) same = same && F.si == A.f[0].si && F.sj == A.f[0].sj && F.sk == A.f[0].sk;
+  auto kern = same ? update_atmos_state_kernel<true> : update_atmos_state_kernel<false>;
+  const size_t smem = sizeof(double) * 2 * AT_TC * (size_t)(A.nz + 1);
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  kern<<<(unsigned)((ncf + AT_TC - 1) / AT_TC), AT_TC * AT_NW, smem, st>>>(A);
+  kern<<<(unsigned)((ncf + AT_TC - 1) / AT_TC), AT_TC * AT_LW, smem, st>>>(A);
   return cudaGetLastError();
 }
 
@@ -417,9 +432,11 @@ extern "C" int shield_update_atmos_state(int nx, int ny, int nz, int hx, int mod
   A.C_LIQ = 4.1855e3;
   A.C_ICE = 1972.0;
   const int64_t ncf = (int64_t)(nx + 2 * hx) * (ny + 2 * hx);
-  const int nk = nz + 1;
-  cudaError_t e = nk <= 96 ? launch_atmos<96>(A, ncf, static_cast<cudaStream_t>(stream))
-                           : launch_atmos<129>(A, ncf, static_cast<cudaStream_t>(stream));
+  if (ncf > INT32_MAX) {
+    shield::set_last_error("shield_update_atmos_state: more than 2^31 - 1 columns");
+    return SHIELD_ELAYOUT;
+  }
+  cudaError_t e = launch_atmos(A, (int)ncf, static_cast<cudaStream_t>(stream));
   if (e != cudaSuccess) {
     shield::set_last_error(std::string("shield_update_atmos_state: ") + cudaGetErrorString(e));
     return SHIELD_ECUDA;
