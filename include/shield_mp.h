@@ -132,6 +132,11 @@ int shield_mp_step(void* handle, const ShieldMpFields* fields, double timestep, 
  * sign of a rounding residue. Agrees with shield_mp_step to round-off. */
 int shield_mp_step_ieee(void* handle, const ShieldMpFields* fields, double timestep, void* stream);
 
+/* shield_mp_step on tendencies that count as zero: their contents are not
+ * read and the whole compute domain of each is written, as prepare_microphysics
+ * followed by shield_mp_step leaves them. Not with de_ice (SHIELD_EINVAL). */
+int shield_mp_step_fresh(void* handle, const ShieldMpFields* fields, double timestep, int precision, void* stream);
+
 int shield_mp_destroy(void* handle);
 
 /* Copies the handle's last error message (NUL terminated) into buf. */

@@ -161,6 +161,7 @@ EXPORTS = (
     "shield_mp_create",
     "shield_mp_step",
     "shield_mp_step_ieee",
+    "shield_mp_step_fresh",
     "shield_mp_destroy",
     "shield_mp_last_error",
     "shield_mp_constants",
@@ -208,6 +209,7 @@ def load():
     vp, i32, dbl = ctypes.c_void_p, ctypes.c_int, ctypes.c_double
     lib.shield_mp_create.argtypes = [ctypes.POINTER(ShieldMpConfig), i32, i32, i32, ShieldField2D, ctypes.POINTER(vp)]
     lib.shield_mp_step.argtypes = [vp, ctypes.POINTER(ShieldMpFields), dbl, i32, vp]
+    lib.shield_mp_step_fresh.argtypes = [vp, ctypes.POINTER(ShieldMpFields), dbl, i32, vp]
     lib.shield_mp_step_ieee.argtypes = [vp, ctypes.POINTER(ShieldMpFields), dbl, vp]
     lib.shield_mp_destroy.argtypes = [vp]
     lib.shield_mp_last_error.argtypes = [vp, ctypes.c_char_p, ctypes.c_size_t]

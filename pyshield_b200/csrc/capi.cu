@@ -111,7 +111,7 @@ namespace {
 // launch also records each sub-step's column flags there; with `ieee` (plain
 // form only) it keeps the reference's rounding.
 int step_impl(Handle* h, const ShieldMpFields* F, double timestep, int precision, int32_t* flags, int64_t nflags,
-              void* stream, bool ieee = false) {
+              void* stream, bool ieee = false, bool fresh = false) {
   if (!h) return fail(nullptr, SHIELD_EINVAL, "null handle");
   if (!F) return fail(h, SHIELD_EINVAL, "null fields");
   if (precision != SHIELD_MP_PLAIN && precision != SHIELD_MP_MIXED)
@@ -163,6 +163,9 @@ int step_impl(Handle* h, const ShieldMpFields* F, double timestep, int precision
                       std::to_string((int64_t)h->K.ntimes * h->ncol));
     A.flags = flags;
   }
+  // de_ice reads and rewrites the incoming tendencies
+  if (fresh && h->K.de_ice) return fail(h, SHIELD_EINVAL, "de_ice needs the incoming tendencies");
+  A.fresh = fresh ? 1 : 0;
   plan_layout(A);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   cudaError_t e = cudaSuccess;
@@ -179,6 +182,11 @@ int step_impl(Handle* h, const ShieldMpFields* F, double timestep, int precision
 
 extern "C" int shield_mp_step(void* handle, const ShieldMpFields* F, double timestep, int precision, void* stream) {
   return step_impl(static_cast<Handle*>(handle), F, timestep, precision, nullptr, 0, stream);
+}
+
+extern "C" int shield_mp_step_fresh(void* handle, const ShieldMpFields* F, double timestep, int precision,
+                                    void* stream) {
+  return step_impl(static_cast<Handle*>(handle), F, timestep, precision, nullptr, 0, stream, false, true);
 }
 
 extern "C" int shield_mp_step_ieee(void* handle, const ShieldMpFields* F, double timestep, void* stream) {

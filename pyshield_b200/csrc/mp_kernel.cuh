@@ -1088,6 +1088,11 @@ SHD int out_mode(const MpConst& K, int o) {
   return m;
 }
 
+// tendency of a step that starts from zero tendencies
+SHD double fresh_tendency(int mode, bool k1, double v) {
+  return (mode == OM_SET) ? v : (mode == OM_ADD || (mode == OM_ADD_K1 && k1)) ? __dadd_rn(0.0, v) : 0.0;
+}
+
 template <class LY>
 SHD void stage_out(const MpArgs& A, const double* sm, int64_t c0) {
   constexpr int RP = LY::RP, G = LY::G;
@@ -1101,16 +1106,22 @@ SHD void stage_out(const MpArgs& A, const double* sm, int64_t c0) {
     const int64_t oq = c0 + M.g + M.k * A.ncol;
     if (!M.ok) return;
     const bool k1 = M.k >= 1;  // the winds' tendencies are written below the top level
+    if (A.fresh) {
 #pragma unroll
-    for (int n = 0; n < OUT_W; ++n) {
-      const int m = out_mode(K, n);
-      old[n] = (m == OM_ADD || (m == OM_ADD_K1 && k1)) ? A.out[n].p[o] : 0.0;
-    }
+      for (int n = 0; n < OUT_W; ++n)
+        A.out[n].p[o] = fresh_tendency(out_mode(K, n), k1, sm[(n * G + M.g) * RP + M.k]);
+    } else {
 #pragma unroll
-    for (int n = 0; n < OUT_W; ++n) {
-      const int m = out_mode(K, n);
-      const double v = sm[(n * G + M.g) * RP + M.k];
-      if (m == OM_SET || m == OM_ADD || (m == OM_ADD_K1 && k1)) A.out[n].p[o] = (m == OM_SET) ? v : old[n] + v;
+      for (int n = 0; n < OUT_W; ++n) {
+        const int m = out_mode(K, n);
+        old[n] = (m == OM_ADD || (m == OM_ADD_K1 && k1)) ? A.out[n].p[o] : 0.0;
+      }
+#pragma unroll
+      for (int n = 0; n < OUT_W; ++n) {
+        const int m = out_mode(K, n);
+        const double v = sm[(n * G + M.g) * RP + M.k];
+        if (m == OM_SET || m == OM_ADD || (m == OM_ADD_K1 && k1)) A.out[n].p[o] = (m == OM_SET) ? v : old[n] + v;
+      }
     }
     if (out_mode(K, OUT_W) == OM_SET) A.out[OUT_W].p[o] = sm[(OUT_W * G + M.g) * RP + M.k];
     A.out[OUT_QAZ].p[oq] = sm[(OUT_QAZ * G + M.g) * RP + M.k];
@@ -1125,7 +1136,9 @@ SHD void stage_out(const MpArgs& A, const double* sm, int64_t c0) {
     const Fld3 F = A.out[o];
     const bool kf = F.sk == 1;
     const int lev = kf ? M.kk : M.k;
-    if (!(kf ? M.okk : M.ok) || (m == OM_ADD_K1 && lev < 1)) m = OM_SKIP;
+    const bool fresh = A.fresh && o < OUT_W;
+    if (!(kf ? M.okk : M.ok) || (!fresh && m == OM_ADD_K1 && lev < 1)) m = OM_SKIP;
+    else if (fresh) m = OM_SET;
     mode[o] = m;
     dst[o] = kf ? F.p + M.ik * F.si + M.jk * F.sj + M.kk : F.p + M.i * F.si + M.j * F.sj + (int64_t)M.k * F.sk;
     old[o] = (m == OM_ADD || m == OM_ADD_K1) ? *dst[o] : 0.0;
@@ -1134,7 +1147,8 @@ SHD void stage_out(const MpArgs& A, const double* sm, int64_t c0) {
   for (int o = 0; o < N_OUT; ++o) {
     if (mode[o] == OM_SKIP) continue;
     const bool kf = A.out[o].sk == 1;
-    const double v = kf ? sm[(o * G + M.gk) * RP + M.kk] : sm[(o * G + M.g) * RP + M.k];
+    double v = kf ? sm[(o * G + M.gk) * RP + M.kk] : sm[(o * G + M.g) * RP + M.k];
+    if (A.fresh && o < OUT_W) v = fresh_tendency(out_mode(K, o), (kf ? M.kk : M.k) >= 1, v);
     *dst[o] = (mode[o] == OM_SET) ? v : old[o] + v;
   }
 }

@@ -100,6 +100,7 @@ struct MpArgs {
   int same_strides;
   Fld3 in[N_IN];
   Fld3 out[N_OUT];
+  int fresh;  // the tendencies count as zero on entry: written whole, not added to
   Fld2 land, area;
   double *rain, *snow, *ice, *graupel;  // (ncol,) surface precipitation [mm/day]; may be null
   int* err;                             // device error word

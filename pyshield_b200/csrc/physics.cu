@@ -98,31 +98,37 @@ __device__ __forceinline__ double np_min(double a, double b) { return a <= b ? a
 //                   prepare_microphysics; del_gz into shared memory;
 //   D  (one warp)   get_phi_fv3's bottom-up sum into shared memory; then
 //      (all warps)  phii, del_gz, phil and prepare_microphysics' dz.
+// SAME: every field has one set of strides (NDSL storages of one shape), so
+// a level has one offset instead of 31.
+// Bound by memory latency and by many short (256 B) write streams. Shapes
+// (level warps, blocks per SM; ms of the launch at C96 L79, zeroing the ten
+// tendencies): 8, 2 with an offset per field 0.502; one offset and 8, 2
+// 0.499; 16, 2 (64 registers) 0.475. Without the zeroing (Physics.__call__,
+// whose step writes the tendencies anew) 0.310.
+constexpr int PRE_MINB = 2;
 constexpr int TC = 32;
-constexpr int NWB = 8;
+constexpr int NWB = 16;
 
-template <int NKMAX>
-struct PreSmem {
-  double ph[NKMAX][TC];  // phase A: delz * GRAV; B: statein's phii
-  double p[NKMAX][TC];   // phase A: dpn of the level above; B: prsi
-  double gz[NKMAX][TC];  // phase C: get_phi_fv3's del_gz
-};
-
-// Two blocks (16 warps) per SM: the kernel waits on memory, so it needs the
-// resident warps; the fused copy's extra loads would otherwise take the
-// registers of the second block.
-template <int NKMAX, bool FUSED>
-__global__ void __launch_bounds__(TC * NWB, 2) physics_prestep_kernel(const __grid_constant__ PhysArgs A) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  PreSmem<NKMAX>& S = *reinterpret_cast<PreSmem<NKMAX>*>(smem_raw);
-  const int nxf = A.nx + 2 * A.hx, nyf = A.ny + 2 * A.hx;
-  const int64_t ncf = (int64_t)nxf * nyf;
+template <bool FUSED, bool SAME>
+__global__ void __launch_bounds__(TC * NWB, FUSED ? 1 : PRE_MINB)
+    physics_prestep_kernel(const __grid_constant__ PhysArgs A) {
+  extern __shared__ double smem[];
+  const int nxf = A.nx + 2 * A.hx;
+  const int ncf = nxf * (A.ny + 2 * A.hx);
   const int nk = A.nz + 1;
   const F3* f = A.f;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int64_t c = (int64_t)blockIdx.x * TC + lane;
+  // rows of nk levels: phase A's delz * GRAV, then statein's phii, then
+  // get_phi_fv3's; phase A's dpn of the level above, then prsi; get_phi_fv3's
+  // del_gz
+  double* const sph = smem + lane;
+  double* const sp = sph + (size_t)nk * TC;
+  double* const sgz = sp + (size_t)nk * TC;
+  const int c = blockIdx.x * TC + lane;
   const bool live = c < ncf;
-  const int64_t i = live ? c % nxf - A.hx : 0, j = live ? c / nxf - A.hx : 0;
+  const int i = live ? c % nxf - A.hx : 0, j = live ? c / nxf - A.hx : 0;
+  const int64_t o0 = i * f[PHII].si + j * f[PHII].sj, okk = f[PHII].sk;
+  auto at = [&](const F3& F, int k) -> double& { return SAME ? F.p[o0 + k * okk] : F.at(i, j, k); };
   const bool compute = live && i >= 0 && j >= 0 && i < A.nx && j < A.ny;
   const bool halo = live && !compute;
   // With the fused copy, DycoreToPhysics' domain -- the compute domain plus
@@ -133,9 +139,9 @@ __global__ void __launch_bounds__(TC * NWB, 2) physics_prestep_kernel(const __gr
   const bool strip = FUSED && halo && i >= 0 && j >= 0 && i <= A.nx && j <= A.ny;
   auto rd = [&](int pf, int df, int k) -> double {
     if constexpr (FUSED) {
-      if (k < A.nz && (compute || strip)) return A.dsrc[df].at(i, j, k);
+      if (k < A.nz && (compute || strip)) return at(A.dsrc[df], k);
     }
-    return f[pf].at(i, j, k);
+    return at(f[pf], k);
   };
 
   // ---- A: statein's prelude (PARALLEL interval(...)): tracers * delp, dpn
@@ -145,16 +151,16 @@ __global__ void __launch_bounds__(TC * NWB, 2) physics_prestep_kernel(const __gr
         // the copied fields statein leaves alone, moved here where the
         // level loop has few loads of its own
         if (k < nk - 1) {
-          const double cz = A.dsrc[D_DELZ].at(i, j, k), ca = A.dsrc[D_QCLD].at(i, j, k);
-          const double cu = A.dsrc[D_UA].at(i, j, k), cv = A.dsrc[D_VA].at(i, j, k), cw = A.dsrc[D_W].at(i, j, k);
-          A.ddst[D_DELZ].at(i, j, k) = cz;
-          A.ddst[D_QCLD].at(i, j, k) = ca;
-          A.ddst[D_UA].at(i, j, k) = cu;
-          A.ddst[D_VA].at(i, j, k) = cv;
-          A.ddst[D_W].at(i, j, k) = cw;
+          const double cz = at(A.dsrc[D_DELZ], k), ca = at(A.dsrc[D_QCLD], k);
+          const double cu = at(A.dsrc[D_UA], k), cv = at(A.dsrc[D_VA], k), cw = at(A.dsrc[D_W], k);
+          at(A.ddst[D_DELZ], k) = cz;
+          at(A.ddst[D_QCLD], k) = ca;
+          at(A.ddst[D_UA], k) = cu;
+          at(A.ddst[D_VA], k) = cv;
+          at(A.ddst[D_W], k) = cw;
         }
       }
-      if (k < nk - 1) S.ph[k][lane] = rd(DELZ, D_DELZ, k) * A.GRAV;
+      if (k < nk - 1) sph[k * TC] = rd(DELZ, D_DELZ, k) * A.GRAV;
       const double dp0 = rd(DELP, D_DELP, k);
       double q[N_TRACER];
 #pragma unroll
@@ -162,33 +168,33 @@ __global__ void __launch_bounds__(TC * NWB, 2) physics_prestep_kernel(const __gr
       // q[1..5]: ql qr qi qs qg (the argument order qliquid, qrain, qice, qsnow, qgraupel)
       const double dpn = A.nwat == 6 ? dp0 - q[1] - q[2] - q[3] - q[4] - q[5] : dp0;
       if (k < nk - 1) {
-        S.p[k + 1][lane] = dpn;
+        sp[(k + 1) * TC] = dpn;
       } else {
         // the extra level: mass-weighted tracers and thickness, no division
 #pragma unroll
-        for (int t = 0; t < N_TRACER; ++t) f[QV + t].at(i, j, k) = q[t];
-        f[DELP].at(i, j, k) = dpn;
+        for (int t = 0; t < N_TRACER; ++t) at(f[QV + t], k) = q[t];
+        at(f[DELP], k) = dpn;
       }
     } else if (halo) {
-      S.p[k][lane] = f[PRSI].at(i, j, k);
-      S.ph[k][lane] = f[PHII].at(i, j, k);
+      sp[k * TC] = at(f[PRSI], k);
+      sph[k * TC] = at(f[PHII], k);
     }
   }
   __syncthreads();
   // ---- B: statein's running sums, in the reference's order (two warps)
   if (w == 0 && compute) {
     double ph = 0.0;
-    S.ph[nk - 1][lane] = ph;
+    sph[(nk - 1) * TC] = ph;
     for (int k = nk - 2; k >= 0; --k) {  // BACKWARD: phii[k] = phii[k + 1] - delz * GRAV
-      ph = ph - S.ph[k][lane];
-      S.ph[k][lane] = ph;
+      ph = ph - sph[k * TC];
+      sph[k * TC] = ph;
     }
   } else if (w == 1 && compute) {
     double p = A.ptop;  // FORWARD: prsi[k] = prsi[k - 1] + delp[k - 1]
-    S.p[0][lane] = p;
+    sp[0 * TC] = p;
     for (int k = 1; k < nk; ++k) {
-      p = p + S.p[k][lane];
-      S.p[k][lane] = p;
+      p = p + sp[k * TC];
+      sp[k * TC] = p;
     }
   }
   __syncthreads();
@@ -198,10 +204,10 @@ __global__ void __launch_bounds__(TC * NWB, 2) physics_prestep_kernel(const __gr
   // between two loads would make each group of loads wait for the last.
   for (int k = w; k < nk; k += NWB) {
     if (compute) {
-      const double p = S.p[k][lane];
+      const double p = sp[k * TC];
       if (k == nk - 1) {
-        f[PRSI].at(i, j, k) = p;
-        f[PRSIK].at(i, j, k) = exp(A.KAPPA * log(p)) * A.pk0inv;
+        at(f[PRSI], k) = p;
+        at(f[PRSIK], k) = exp(A.KAPPA * log(p)) * A.pk0inv;
         continue;
       }
       // loads
@@ -213,8 +219,8 @@ __global__ void __launch_bounds__(TC * NWB, 2) physics_prestep_kernel(const __gr
       const double pt = rd(PT, D_PT, k);
       const double om = (A.prepare || FUSED) ? rd(OMGA, D_OMGA, k) : 0.0;
       // statein
-      const double pn = S.p[k + 1][lane];
-      const double ph_k = S.ph[k][lane], ph1 = S.ph[k + 1][lane];
+      const double pn = sp[(k + 1) * TC];
+      const double ph_k = sph[k * TC], ph1 = sph[(k + 1) * TC];
 #pragma unroll
       for (int t = 0; t < N_TRACER; ++t) q[t] = q[t] * dp0;
       const double dpn = A.nwat == 6 ? dp0 - q[1] - q[2] - q[3] - q[4] - q[5] : dp0;
@@ -229,25 +235,25 @@ __global__ void __launch_bounds__(TC * NWB, 2) physics_prestep_kernel(const __gr
       d = np_max(d, p + 0.01 * dm);
       const double tv = 1.0 + A.ZVIR * np_max(0.0, qv);
       const double gz = (ph_k - ph1) / (pt * tv);
-      S.gz[k][lane] = gz * pt * tv;
+      sgz[k * TC] = gz * pt * tv;
       // stores
-      f[PRSI].at(i, j, k) = p;
-      f[PRSIK].at(i, j, k) = k == 0 ? A.pktop : log(p);
+      at(f[PRSI], k) = p;
+      at(f[PRSIK], k) = k == 0 ? A.pktop : log(p);
 #pragma unroll
-      for (int t = 0; t < N_TRACER; ++t) f[QV + t].at(i, j, k) = q[t];
-      f[TKE].at(i, j, k) = tke / dpn;
-      f[DM].at(i, j, k) = dm;
-      f[DELP].at(i, j, k) = d;
-      f[DELPRSI].at(i, j, k) = pn - p;
+      for (int t = 0; t < N_TRACER; ++t) at(f[QV + t], k) = q[t];
+      at(f[TKE], k) = tke / dpn;
+      at(f[DM], k) = dm;
+      at(f[DELP], k) = d;
+      at(f[DELPRSI], k) = pn - p;
       if constexpr (FUSED) {
-        A.ddst[D_PT].at(i, j, k) = pt;
-        A.ddst[D_OMGA].at(i, j, k) = om;
+        at(A.ddst[D_PT], k) = pt;
+        at(A.ddst[D_OMGA], k) = om;
       }
       if (A.prepare) {
-        f[WMP].at(i, j, k) = -om * (1.0 + A.ZVIR * qv) * pt / d * A.RDGAS_RGRAV;
+        at(f[WMP], k) = -om * (1.0 + A.ZVIR * qv) * pt / d * A.RDGAS_RGRAV;
 #pragma unroll
         for (int t = 0; t < 10; ++t)
-          if (f[TEND0 + t].p) f[TEND0 + t].at(i, j, k) = 0.0;
+          if (f[TEND0 + t].p) at(f[TEND0 + t], k) = 0.0;
       }
     } else if (halo && k < nk - 1) {
       const double pt = rd(PT, D_PT, k);
@@ -256,14 +262,14 @@ __global__ void __launch_bounds__(TC * NWB, 2) physics_prestep_kernel(const __gr
         // DycoreToPhysics' copy of this interface column (a few columns:
         // one field at a time, to keep the registers for the compute path)
 #pragma unroll 1
-        for (int d = 0; d < N_D2P; ++d) A.ddst[d].at(i, j, k) = A.dsrc[d].at(i, j, k);
+        for (int d = 0; d < N_D2P; ++d) at(A.ddst[d], k) = at(A.dsrc[d], k);
       }
-      const double p = S.p[k][lane], pn = S.p[k + 1][lane];
-      const double ph_k = S.ph[k][lane], ph1 = S.ph[k + 1][lane];
+      const double p = sp[k * TC], pn = sp[(k + 1) * TC];
+      const double ph_k = sph[k * TC], ph1 = sph[(k + 1) * TC];
       const double tv = 1.0 + A.ZVIR * np_max(0.0, qv);
-      f[DELPRSI].at(i, j, k) = pn - p;
+      at(f[DELPRSI], k) = pn - p;
       const double gz = (ph_k - ph1) / (pt * tv);
-      S.gz[k][lane] = gz * pt * tv;
+      sgz[k * TC] = gz * pt * tv;
     }
   }
   __syncthreads();
@@ -272,10 +278,10 @@ __global__ void __launch_bounds__(TC * NWB, 2) physics_prestep_kernel(const __gr
   // then phii, del_gz, phil and prepare_microphysics' dz from all warps
   if (w == 0 && live) {
     double ph = 0.0;
-    S.ph[nk - 1][lane] = ph;
+    sph[(nk - 1) * TC] = ph;
     for (int k = nk - 2; k >= 0; --k) {
-      const double phn = ph + S.gz[k][lane];
-      S.ph[k][lane] = phn;
+      const double phn = ph + sgz[k * TC];
+      sph[k * TC] = phn;
       ph = phn;
     }
   }
@@ -284,27 +290,30 @@ __global__ void __launch_bounds__(TC * NWB, 2) physics_prestep_kernel(const __gr
     const bool prep = compute && A.prepare;
     for (int k = w; k < nk; k += NWB) {
       if (k == nk - 1) {
-        f[PHII].at(i, j, k) = 0.0;
+        at(f[PHII], k) = 0.0;
         continue;
       }
-      const double g = S.gz[k][lane];
-      const double ph = S.ph[k + 1][lane], phn = S.ph[k][lane];
-      f[DELGZ].at(i, j, k) = g;
-      f[PHIL].at(i, j, k) = 0.5 * (ph + ph + g);
-      f[PHII].at(i, j, k) = phn;
-      if (prep) f[DZ].at(i, j, k) = (ph - phn) * A.RGRAV;
+      const double g = sgz[k * TC];
+      const double ph = sph[(k + 1) * TC], phn = sph[k * TC];
+      at(f[DELGZ], k) = g;
+      at(f[PHIL], k) = 0.5 * (ph + ph + g);
+      at(f[PHII], k) = phn;
+      if (prep) at(f[DZ], k) = (ph - phn) * A.RGRAV;
     }
   }
 }
 
-template <int NKMAX>
-cudaError_t launch_prestep(const PhysArgs& A, int64_t ncf, cudaStream_t st) {
-  const size_t smem = sizeof(PreSmem<NKMAX>);
-  auto kern = A.fused ? physics_prestep_kernel<NKMAX, true> : physics_prestep_kernel<NKMAX, false>;
+cudaError_t launch_prestep(const PhysArgs& A, int ncf, cudaStream_t st) {
+  bool same = true;
+  auto like = [&](const F3& F) { return !F.p || (F.si == A.f[PHII].si && F.sj == A.f[PHII].sj && F.sk == A.f[PHII].sk); };
+  for (const F3& F : A.f) same = same && like(F);
+  for (int d = 0; A.fused && d < N_D2P; ++d) same = same && like(A.dsrc[d]) && like(A.ddst[d]);
+  auto kern = A.fused ? (same ? physics_prestep_kernel<true, true> : physics_prestep_kernel<true, false>)
+                      : (same ? physics_prestep_kernel<false, true> : physics_prestep_kernel<false, false>);
+  const size_t smem = sizeof(double) * 3 * TC * (size_t)(A.nz + 1);
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  const int64_t nblk = (ncf + TC - 1) / TC;
-  kern<<<(unsigned)nblk, TC * NWB, smem, st>>>(A);
+  kern<<<(unsigned)((ncf + TC - 1) / TC), TC * NWB, smem, st>>>(A);
   return cudaGetLastError();
 }
 
@@ -371,8 +380,11 @@ int prestep_impl(int nx, int ny, int nz, int hx, int nwat, double ptop, int flag
   A.pk0inv = std::pow(1.0 / p00, A.KAPPA);
   const int64_t ncf = (int64_t)(nx + 2 * hx) * (ny + 2 * hx);
   const cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const int nk = nz + 1;
-  cudaError_t e = nk <= 96 ? launch_prestep<96>(A, ncf, st) : launch_prestep<129>(A, ncf, st);
+  if (ncf > INT32_MAX) {
+    shield::set_last_error("shield_physics_prestep: more than 2^31 - 1 columns");
+    return SHIELD_ELAYOUT;
+  }
+  cudaError_t e = launch_prestep(A, (int)ncf, st);
   if (e != cudaSuccess) {
     shield::set_last_error(std::string("shield_physics_prestep: ") + cudaGetErrorString(e));
     return SHIELD_ECUDA;

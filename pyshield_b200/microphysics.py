@@ -148,6 +148,17 @@ class Microphysics:
         )
         check(rc, self._handle, "shield_mp_step")
 
+    def step_fresh(self, state, timestep, stream=None):
+        """``__call__`` on tendencies that count as zero: they are written
+        whole and their contents are not read (what zeroing them and
+        ``__call__`` leave). Not with ``de_ice``, which reads ``qi_dt``."""
+        self._build_fields(state)
+        rc = load().shield_mp_step_fresh(
+            self._handle, ctypes.byref(self._fields), float(timestep), _PRECISION[self.precision],
+            ctypes.c_void_p(_current_stream(stream)),
+        )
+        check(rc, self._handle, "shield_mp_step_fresh")
+
     def step_with_flags(self, state, timestep, stream=None):
         """``__call__`` (plain FP64 form) that also returns the step's column
         branch flags: an int32 tensor (ntimes, ny, nx) whose bits are the
