@@ -129,8 +129,9 @@ int shield_mp_step(void* handle, const ShieldMpFields* fields, double timestep, 
 /* shield_mp_step in the plain form with the rounding of every operation of
  * the reference's expressions (CUDA's exp, log and pow, IEEE division): the
  * forward step of a differentiated window, whose branches may hang on the
- * sign of a rounding residue. Agrees with shield_mp_step to round-off. */
-int shield_mp_step_ieee(void* handle, const ShieldMpFields* fields, double timestep, void* stream);
+ * sign of a rounding residue. Agrees with shield_mp_step to round-off; with
+ * `fresh`, the tendencies count as zero (shield_mp_step_fresh). */
+int shield_mp_step_ieee(void* handle, const ShieldMpFields* fields, double timestep, int fresh, void* stream);
 
 /* shield_mp_step on tendencies that count as zero: their contents are not
  * read and the whole compute domain of each is written, as prepare_microphysics

@@ -210,7 +210,7 @@ def load():
     lib.shield_mp_create.argtypes = [ctypes.POINTER(ShieldMpConfig), i32, i32, i32, ShieldField2D, ctypes.POINTER(vp)]
     lib.shield_mp_step.argtypes = [vp, ctypes.POINTER(ShieldMpFields), dbl, i32, vp]
     lib.shield_mp_step_fresh.argtypes = [vp, ctypes.POINTER(ShieldMpFields), dbl, i32, vp]
-    lib.shield_mp_step_ieee.argtypes = [vp, ctypes.POINTER(ShieldMpFields), dbl, vp]
+    lib.shield_mp_step_ieee.argtypes = [vp, ctypes.POINTER(ShieldMpFields), dbl, i32, vp]
     lib.shield_mp_destroy.argtypes = [vp]
     lib.shield_mp_last_error.argtypes = [vp, ctypes.c_char_p, ctypes.c_size_t]
     lib.shield_mp_constants.argtypes = [vp, dbl, ctypes.POINTER(ctypes.c_double), i32]

@@ -36,7 +36,7 @@ from ._lib import (
     load,
 )
 from .microphysics import _current_stream
-from .quantity import field2d, field3d
+from .quantity import field2d, field3d, set_fields3d
 
 # pt qvapor qliquid qrain qice qsnow qgraupel qcld ua va delprsi delz wmp, and the accumulator
 STATE = MP_STATE_FIELDS + ("qaz",)
@@ -52,7 +52,7 @@ def _empty3(like):
     import torch
 
     nx, ny, nz = like.shape
-    return torch.zeros((nz, ny, nx), dtype=torch.float64, device=like.device).permute(2, 1, 0)
+    return torch.empty((nz, ny, nx), dtype=torch.float64, device=like.device).permute(2, 1, 0)
 
 
 def _check_state(mp, state):
@@ -66,8 +66,7 @@ def _check_state(mp, state):
 def _state_fields(mp, state, land):
     F = ShieldMpFields()
     ext = (mp.nx, mp.ny, mp.nz)
-    for name, t in zip(MP_STATE_FIELDS, state):
-        setattr(F, name, field3d(t, ext))
+    set_fields3d(F, state[:len(MP_STATE_FIELDS)], ext)
     F.land = field2d(land, (mp.nx, mp.ny))
     return F
 
@@ -89,10 +88,15 @@ def step_forward(mp, state, land, timestep, stream=None, tendencies=None):
     w_out.copy_(state[STATE.index("wmp")])
     F.wmp = field3d(w_out, (mp.nx, mp.ny, mp.nz))
     tend = [_empty3(state[0]) for _ in MP_TENDENCY_FIELDS]
-    for name, t in zip(MP_TENDENCY_FIELDS, tend):
-        if tendencies is not None and tendencies.get(name) is not None:
-            t.copy_(tendencies[name])
-        setattr(F, name, field3d(t, (mp.nx, mp.ny, mp.nz)))
+    # without incoming tendencies the step writes them whole (de_ice reads qi_dt)
+    fresh = tendencies is None and not mp._cfg.de_ice
+    if not fresh:
+        for name, t in zip(MP_TENDENCY_FIELDS, tend):
+            if tendencies is not None and tendencies.get(name) is not None:
+                t.copy_(tendencies[name])
+            else:
+                t.zero_()
+    set_fields3d(F, tend, (mp.nx, mp.ny, mp.nz), len(MP_STATE_FIELDS))
     if tendencies is not None:
         # de_ice writes the step's input qi and qs in place
         keep_q = []
@@ -106,7 +110,7 @@ def step_forward(mp, state, land, timestep, stream=None, tendencies=None):
     F.rain, F.snow, F.ice, F.graupel = base, base + plane, base + 2 * plane, base + 3 * plane
     # the form that keeps the reference's rounding: a window's branches may
     # hang on the sign of a rounding residue (csrc/mp_ieee.cu)
-    rc = load().shield_mp_step_ieee(mp._handle, ctypes.byref(F), float(timestep),
+    rc = load().shield_mp_step_ieee(mp._handle, ctypes.byref(F), float(timestep), int(fresh),
                                     ctypes.c_void_p(_current_stream(stream)))
     check(rc, mp._handle, "shield_mp_step_ieee")
     qaz = mp.get_qaz().permute(2, 1, 0)
@@ -141,8 +145,7 @@ def step_vjp(mp, state, land, cot, timestep, stream=None, tendencies=None):
         setattr(C, name, cc.data_ptr())
     G = ShieldMpGradients()
     grads = [_empty3(state[0]) for _ in STATE]
-    for name, g in zip(STATE, grads):
-        setattr(G, name, field3d(g, ext))
+    set_fields3d(G, grads, ext)
     rc = load().shield_mp_step_vjp(mp._handle, ctypes.byref(F), ctypes.byref(C), ctypes.byref(G), float(timestep),
                                    ctypes.c_void_p(_current_stream(stream)))
     check(rc, mp._handle, "shield_mp_step_vjp")

@@ -23,9 +23,9 @@ stencils) for the caller's horizontal step.
 import ctypes
 
 from . import constants as C
-from ._lib import SHIELD_UAS_APPLY, SHIELD_UAS_DYCORE_ONLY, ShieldField3D, check, load
+from ._lib import SHIELD_UAS_APPLY, SHIELD_UAS_DYCORE_ONLY, check, load
 from .microphysics import _current_stream
-from .quantity import field3d
+from .quantity import field3d, fields3d
 
 
 def _domain(q):
@@ -51,10 +51,7 @@ def update_physics_state_with_tendencies(
         physics_updated_qsnow, physics_updated_qgraupel, physics_updated_cloud_fraction, physics_updated_pt,
         physics_updated_ua, physics_updated_va,
     )
-    arr = ShieldField3D * 10
-    s = arr(*[field3d(q, ext) for q in state])
-    t = arr(*[field3d(q, ext) for q in tend])
-    o = arr(*[field3d(q, ext) for q in out])
+    s, t, o = fields3d(state, ext), fields3d(tend, ext), fields3d(out, ext)
     rc = load().shield_update_physics_state(nx, ny, nz, s, t, o, float(dt), ctypes.c_void_p(_current_stream(stream)))
     check(rc, None, "shield_update_physics_state")
 
@@ -107,7 +104,7 @@ class UpdateAtmosphereState:
             d.qvapor, d.qliquid, d.qrain, d.qsnow, d.qice, d.qgraupel, p.prsi, d.delp, d.pt, d.pe, d.peln, d.pk,
             d.ua, d.va,
         )
-        arr = (ShieldField3D * len(fields))(*[field3d(q, ext) for q in fields])
+        arr = fields3d(fields, ext)
         # halo reach of fill_gfs_delp: the full domain around the compute domain
         for q in (p.physics_updated_specific_humidity, d.qvapor, d.delp):
             org = tuple(getattr(q, "origin", (0, 0, 0)))
@@ -170,9 +167,8 @@ class DycoreToPhysics:
         if self._dycore_only:
             return
         ext = (self.nx + 1, self.ny + 1, self.nz)
-        arr = ShieldField3D * len(D2P_FIELDS)
-        src = arr(*[field3d(getattr(dycore_state, f), ext) for f in D2P_FIELDS])
-        dst = arr(*[field3d(getattr(physics_state, f), ext) for f in D2P_FIELDS])
+        src = fields3d([getattr(dycore_state, f) for f in D2P_FIELDS], ext)
+        dst = fields3d([getattr(physics_state, f) for f in D2P_FIELDS], ext)
         rc = load().shield_copy_dycore_to_physics(self.nx, self.ny, self.nz, src, dst,
                                                   ctypes.c_void_p(_current_stream(stream)))
         check(rc, None, "shield_copy_dycore_to_physics")

@@ -189,8 +189,8 @@ extern "C" int shield_mp_step_fresh(void* handle, const ShieldMpFields* F, doubl
   return step_impl(static_cast<Handle*>(handle), F, timestep, precision, nullptr, 0, stream, false, true);
 }
 
-extern "C" int shield_mp_step_ieee(void* handle, const ShieldMpFields* F, double timestep, void* stream) {
-  return step_impl(static_cast<Handle*>(handle), F, timestep, SHIELD_MP_PLAIN, nullptr, 0, stream, true);
+extern "C" int shield_mp_step_ieee(void* handle, const ShieldMpFields* F, double timestep, int fresh, void* stream) {
+  return step_impl(static_cast<Handle*>(handle), F, timestep, SHIELD_MP_PLAIN, nullptr, 0, stream, true, fresh != 0);
 }
 
 extern "C" int shield_mp_step_flags(void* handle, const ShieldMpFields* F, double timestep, int32_t* flags,

@@ -24,7 +24,7 @@ import ctypes
 
 from . import _lib
 from ._lib import SHIELD_MP_MIXED, SHIELD_MP_PLAIN, ShieldMpFields, check, load, make_config
-from .quantity import field2d, field3d
+from .quantity import field2d, set_fields3d
 
 _PRECISION = {"plain": SHIELD_MP_PLAIN, "fp64": SHIELD_MP_PLAIN, "mixed": SHIELD_MP_MIXED}
 
@@ -127,9 +127,8 @@ class Microphysics:
 
     def _build_fields(self, state):
         F = self._fields
-        ext3 = (self.nx, self.ny, self.nz)
-        for name in _lib.MP_STATE_FIELDS + _lib.MP_TENDENCY_FIELDS:
-            setattr(F, name, field3d(getattr(state, name), ext3))
+        names = _lib.MP_STATE_FIELDS + _lib.MP_TENDENCY_FIELDS
+        set_fields3d(F, [getattr(state, name) for name in names], (self.nx, self.ny, self.nz))
         F.land = field2d(state.land, (self.nx, self.ny))
         base = self._precip.data_ptr()
         plane = self.nx * self.ny * 8

@@ -38,11 +38,14 @@ from ._lib import SHIELD_PHYS_PREPARE_MICROPHYSICS, ShieldPhysicsFields, check, 
 from .coupling import D2P_FIELDS, update_physics_state_with_tendencies
 from .grid import X_DIM, Y_DIM, Z_DIM, Z_INTERFACE_DIM
 from .microphysics import Microphysics, MicrophysicsState, _current_stream
-from .quantity import Quantity, field3d
+from .quantity import Quantity, fields3d, set_fields3d
 
 _XYZ = [X_DIM, Y_DIM, Z_DIM]
 _XYZI = [X_DIM, Y_DIM, Z_INTERFACE_DIM]
 _XY = [X_DIM, Y_DIM]
+
+
+_FULL_DOMAIN = ("phii", "prsi", "delprsi", "del_gz", "phil", "pt", "qvapor")
 
 
 def _field(name, dims, units):
@@ -234,25 +237,36 @@ class Physics:
         src = {
             "prsik": self._prsik, "dm": self._dm3d, "del_gz": self._del_gz,
         }
+        skip = set()
+        if mp is None or not zero_tendencies:
+            skip.update(_lib.MP_TENDENCY_FIELDS)
+        if not self._gfs_microphysics:
+            skip.update(("omga", "dz", "wmp"))
+        qs = []
         for name in _lib.PHYS_FIELDS:
             if name in src:
                 q = src[name]
             elif name in _lib.MP_TENDENCY_FIELDS:
-                if mp is None or not zero_tendencies:
-                    setattr(F, name, _lib.ShieldField3D())
-                    continue
-                q = getattr(mp, name)
-            elif name in ("omga", "dz", "wmp") and not self._gfs_microphysics:
-                setattr(F, name, _lib.ShieldField3D())
-                continue
+                q = None if name in skip else getattr(mp, name)
             else:
-                q = getattr(ps, name)
-            if name in ("phii", "prsi", "delprsi", "del_gz", "phil", "pt", "qvapor"):
+                q = None if name in skip else getattr(ps, name)
+            if name in _FULL_DOMAIN:
                 # read or written on the full domain by get_prs_fv3 / get_phi_fv3
-                org = tuple(getattr(q, "origin", (0, 0, 0)))
+                org = getattr(q, "origin", (0, 0, 0))
                 if org[0] < h or org[1] < h:
                     raise ValueError(f"{name}: get_prs_fv3/get_phi_fv3 need the halo of the full domain")
-            setattr(F, name, field3d(q, ext))
+            qs.append(q)
+        # runs of present fields; an absent one is a null pointer
+        at = 0
+        while at < len(qs):
+            end = at
+            while end < len(qs) and qs[end] is not None:
+                end += 1
+            if end > at:
+                set_fields3d(F, qs[at:end], ext, at)
+            if end < len(qs):
+                setattr(F, _lib.PHYS_FIELDS[end], _lib.ShieldField3D())
+            at = end + 1
         return F
 
     def prestep(self, physics_state, stream=None, dycore_state=None):
@@ -277,9 +291,8 @@ class Physics:
             check(rc, None, "shield_physics_prestep")
             return
         ext = (self.nx + 1, self.ny + 1, self.nz)
-        arr = _lib.ShieldField3D * len(D2P_FIELDS)
-        src = arr(*[field3d(getattr(dycore_state, f), ext) for f in D2P_FIELDS])
-        dst = arr(*[field3d(getattr(ps, f), ext) for f in D2P_FIELDS])
+        src = fields3d([getattr(dycore_state, f) for f in D2P_FIELDS], ext)
+        dst = fields3d([getattr(ps, f) for f in D2P_FIELDS], ext)
         rc = load().shield_physics_prestep_from_dycore(self.nx, self.ny, self.nz, self.n_halo, self._nwat, self._ptop,
                                                        flags, ctypes.byref(self._fields), src, dst, st)
         check(rc, None, "shield_physics_prestep_from_dycore")

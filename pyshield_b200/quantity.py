@@ -8,7 +8,16 @@ domain. Any object with those three attributes works here, as long as
 element strides are passed to the kernels.
 """
 
+import struct
+
 import numpy as np
+
+try:
+    import torch
+
+    _Tensor, _F64 = torch.Tensor, torch.float64
+except ImportError:  # pragma: no cover
+    _Tensor, _F64 = (), None
 
 from ._lib import ShieldField2D, ShieldField3D
 
@@ -33,17 +42,12 @@ class Quantity:
 
 def _array_info(a):
     """(device pointer, element strides, shape) of a float64 CUDA array."""
-    try:
-        import torch
-
-        if isinstance(a, torch.Tensor):
-            if a.dtype != torch.float64:
-                raise TypeError(f"expected float64 data, got {a.dtype}")
-            if not a.is_cuda:
-                raise TypeError("the microphysics kernels need device (CUDA) arrays")
-            return a.data_ptr(), tuple(a.stride()), tuple(a.shape)
-    except ImportError:  # pragma: no cover
-        pass
+    if isinstance(a, _Tensor):
+        if a.dtype != _F64:
+            raise TypeError(f"expected float64 data, got {a.dtype}")
+        if not a.is_cuda:
+            raise TypeError("the microphysics kernels need device (CUDA) arrays")
+        return a.data_ptr(), tuple(a.stride()), tuple(a.shape)
     cai = getattr(a, "__cuda_array_interface__", None)
     if cai is None:
         raise TypeError(f"{type(a).__name__} is not a CUDA array (no __cuda_array_interface__)")
@@ -94,3 +98,40 @@ def field2d(q, extent=None):
             raise ValueError(f"domain origin {org} extent {ext} exceeds storage {shape}")
     off = org[0] * st[0] + org[1] * st[1]
     return ShieldField2D(ptr + 8 * off, st[0], st[1])
+
+
+def _words3d(qs, ext):
+    """field3d(q, ext) of every quantity in ``qs`` as a flat list of words.
+    A call names 24 to 60 fields, and one ctypes structure per field was most
+    of a small call's time (one C12 tile's step: 107 us a call for 33 us on
+    the GPU; 41 us with the words packed at once)."""
+    nx, ny, nz = ext
+    out = []
+    for q in qs:
+        data = q if isinstance(q, _Tensor) else getattr(q, "data", q)
+        if not (isinstance(data, _Tensor) and data.dtype == _F64 and data.is_cuda and data.dim() == 3):
+            f = field3d(q, ext)
+            out += (f.ptr or 0, f.si, f.sj, f.sk)
+            continue
+        si, sj, sk = data.stride()
+        ni, nj, nk = data.shape
+        oi, oj, ok = getattr(q, "origin", None) or (0, 0, 0)
+        if oi < 0 or oj < 0 or ok < 0 or oi + nx > ni or oj + ny > nj or ok + nz > nk:
+            raise ValueError(f"domain origin {(oi, oj, ok)} extent {tuple(ext)} exceeds storage {(ni, nj, nk)}")
+        out += (data.data_ptr() + 8 * (oi * si + oj * sj + ok * sk), si, sj, sk)
+    return out
+
+
+def fields3d(qs, ext):
+    """An array of ShieldField3D: field3d(q, ext) of every quantity."""
+    words = _words3d(qs, ext)
+    arr = (ShieldField3D * (len(words) // 4))()
+    struct.pack_into(f"{len(words)}q", arr, 0, *words)
+    return arr
+
+
+def set_fields3d(struct_, qs, ext, first=0):
+    """field3d(q, ext) of every quantity into the ShieldField3D members of a
+    structure, from member ``first`` on (they stand one after another)."""
+    words = _words3d(qs, ext)
+    struct.pack_into(f"{len(words)}q", struct_, 32 * first, *words)
