@@ -274,28 +274,35 @@ SHP void revap_racc(const MpConst& K, double dt, double h_var, T& qg, T& qi, T& 
     T dqv = qsat - qv;
     T q_minus = qpz - dqh;
     T q_plus = qpz + dqh;
-    if ((dqv > QVMIN) && (qsat > q_minus)) {
-      T dq;
-      if (qsat > q_plus)
-        dq = qsat - qpz;
-      else
-        dq = qdiv(0.25 * sq(q_minus - qsat), dqh);
-      T qden = qr * den;
-      T t2 = tin * tin;
-      T evap = qdiv(K.crevp[0] * t2 * dq * (K.crevp[1] * qsqrt(qden) + K.crevp[2] * xpowc(qden, 0.725)),
-                    K.crevp[3] * t2 + K.crevp[4] * qsat * den);
-      evap = qmin(qr, qmin(dt * evap, qdiv(dqv, 1.0 + lcpk * dqsdt)));
-      qr = qr - evap;
-      qv = qv + evap;
-      q_liq = q_liq - evap;
-      cvm = cvm_of(K, qv, q_liq, q_sol);
-      tz = tz - qdiv(evap * lhl, cvm);
-    }
-    if ((qr > QRMIN) && (ql > 1.0e-6) && (qsat < q_minus)) {
-      T sink = dt * denfac * K.cracw * xpowc(qr * den, 0.95);
-      sink = qdiv(sink, 1.0 + sink) * ql;
-      ql = ql - sink;
-      qr = qr + sink;
+    // Evaporation needs qsat > q_minus, accretion qsat < q_minus (with the
+    // rain as it came): a level does one of the two, and lanes of either kind
+    // share one evaluation of their powers of the rain's density.
+    const bool evaporates = (dqv > QVMIN) && (qsat > q_minus);
+    const bool accretes = !evaporates && (ql > 1.0e-6) && (qsat < q_minus);
+    if (evaporates || accretes) {
+      const T qden = qr * den;
+      const T pw = xpowc(qden, evaporates ? 0.725 : 0.95);
+      if (evaporates) {
+        T dq;
+        if (qsat > q_plus)
+          dq = qsat - qpz;
+        else
+          dq = qdiv(0.25 * sq(q_minus - qsat), dqh);
+        T t2 = tin * tin;
+        T evap = qdiv(K.crevp[0] * t2 * dq * (K.crevp[1] * qsqrt(qden) + K.crevp[2] * pw),
+                      K.crevp[3] * t2 + K.crevp[4] * qsat * den);
+        evap = qmin(qr, qmin(dt * evap, qdiv(dqv, 1.0 + lcpk * dqsdt)));
+        qr = qr - evap;
+        qv = qv + evap;
+        q_liq = q_liq - evap;
+        cvm = cvm_of(K, qv, q_liq, q_sol);
+        tz = tz - qdiv(evap * lhl, cvm);
+      } else {
+        T sink = dt * denfac * K.cracw * pw;
+        sink = qdiv(sink, 1.0 + sink) * ql;
+        ql = ql - sink;
+        qr = qr + sink;
+      }
     }
   }
 }

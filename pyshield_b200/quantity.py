@@ -102,9 +102,9 @@ def field2d(q, extent=None):
 
 def _words3d(qs, ext):
     """field3d(q, ext) of every quantity in ``qs`` as a flat list of words.
-    A call names 24 to 60 fields, and one ctypes structure per field was most
-    of a small call's time (one C12 tile's step: 107 us a call for 33 us on
-    the GPU; 41 us with the words packed at once)."""
+    A call names 24 to 60 fields, and one ctypes structure per field was much
+    of a small call's time (one C12 tile's step: 51 us of host time for 33 us
+    on the GPU; 39 us with the words packed at once)."""
     nx, ny, nz = ext
     out = []
     for q in qs:
