@@ -60,6 +60,12 @@ struct Column {
     else
       asm volatile("bar.sync %0, %1;" ::"r"(bar), "r"(32 * NW) : "memory");
   }
+  // Orders the column's shared accesses before it against those after it,
+  // where its operations do not: a one-warp column's are shuffles and votes,
+  // which order no memory; every other column's pass a barrier.
+  SHD void order() const {
+    if constexpr (NW == 1) __syncwarp();
+  }
   SHD double* slot() {
     double* s = scr + par * Tiles<NW>::SCR;
     par ^= 1;
@@ -632,6 +638,7 @@ struct PackedColumn {
   }
 
   SHD void sync() const { asm volatile("bar.sync %0, %1;" ::"r"(bar), "r"(T) : "memory"); }
+  SHD void order() const {}  // its operations pass the group's barrier
   SHD double* slot() {
     double* s = scr + par * SCR;
     par ^= 1;
@@ -1174,7 +1181,7 @@ struct StepGeom {
 enum ParkSlot { PK_W, PK_DP1, PK_P1, PK_DZ, PK_DZ1, PK_DENFAC, PK_M1, PK_MP, PK_M1SOL, PK_MPSOL, PK_VTR, PK_VTG, PK_VTS };
 struct LevelStore {
   double* pk;  // this thread's slot
-  double* cv;  // the column's values: fields_init's, written by level 0 and read after the next exchange
+  double* cv;  // the column's values: fields_init's, written by level 0 and read after the next exchange (or order())
   double den;  // density (start of each sub-step)
   SHD double& w() const { return pk[PK_W]; }      // vertical velocity
   SHD double& dp1() const { return pk[PK_DP1]; }  // fields_init
@@ -1287,8 +1294,10 @@ SHD void fields_init(Col& C, const MpConst& K, bool valid, double pt, double qvi
       }
     }
   }
-  // after every read of the borrow's work rows, which these slots overlie
-  // (the exchange above lies between)
+  // After every read of the borrow's work rows, which these slots overlie, and
+  // before any read of the column's values: the exchange above lies between,
+  // and the next one (heights), or the warp's own synchronisation.
+  C.order();
   P.w() = wz;
   P.dp1() = dp1;
   P.p1() = p1;
