@@ -127,10 +127,13 @@ int shield_mp_create(const ShieldMpConfig* cfg, int nx, int ny, int nz, ShieldFi
 int shield_mp_step(void* handle, const ShieldMpFields* fields, double timestep, int precision, void* stream);
 
 /* shield_mp_step in the plain form with the rounding of every operation of
- * the reference's expressions (CUDA's exp, log and pow, IEEE division): the
- * forward step of a differentiated window, whose branches may hang on the
- * sign of a rounding residue. Agrees with shield_mp_step to round-off; with
- * `fresh`, the tendencies count as zero (shield_mp_step_fresh). */
+ * the reference's expressions (CUDA's exp, log, pow and square root; quotients
+ * rounded as IEEE division rounds them, for finite normal divisors and
+ * quotients: a zero, infinite or subnormal divisor, which no column of an
+ * atmosphere has, gives a NaN): the forward step of a differentiated window,
+ * whose branches may hang on the sign of a rounding residue. Agrees with
+ * shield_mp_step to round-off; with `fresh`, the tendencies count as zero
+ * (shield_mp_step_fresh). */
 int shield_mp_step_ieee(void* handle, const ShieldMpFields* fields, double timestep, int fresh, void* stream);
 
 /* shield_mp_step on tendencies that count as zero: their contents are not

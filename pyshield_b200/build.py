@@ -22,7 +22,7 @@ LIB = os.path.join(HERE, "libshield_mp.so")
 # the FP64 throughput probe bench.py uses for the step kernel's FP64 roofline,
 # and the device math the tests measure (not part of the C-ABI)
 PROBE_LIB = os.path.join(HERE, "libshield_probe.so")
-PROBE_UNITS = ("peak.cu", "math_probe.cu")
+PROBE_UNITS = ("peak.cu", "math_probe.cu", "math_probe_ieee.cu")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 COMMON = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-Xcompiler", "-ffp-contract=off",
           "--expt-relaxed-constexpr", "-I", os.path.join(os.path.dirname(HERE), "include")]

@@ -39,7 +39,10 @@ __global__ void math_kernel(int fn, int n, const double* x, const double* y, dou
 // out[i] = function `fn` of (x[i], y[i]) for n elements on `stream`: a / b,
 // sqrt, exp, log, x^y, then wqs1, its derivative, iqs1, its derivative at
 // temperature x and density y.
-extern "C" int shield_probe_math(int fn, int n, const double* x, const double* y, double* out, void* stream) {
+#ifndef PROBE_MATH
+#define PROBE_MATH shield_probe_math
+#endif
+extern "C" int PROBE_MATH(int fn, int n, const double* x, const double* y, double* out, void* stream) {
   if (fn < F_DIV || fn > F_QSI_DT || n < 1 || !x || !y || !out) return -1;
   ShieldMpConfig cfg;
   std::memset(&cfg, 0, sizeof(cfg));

@@ -12,7 +12,7 @@
 // outputs do not see this: plain and IEEE forms agree to 1e-14.
 //
 // Division is the branch-free quotient of mp_math.cuh, which rounds as IEEE
-// division does.
+// division does for the finite normal divisors and quotients of the step.
 #define SHIELD_IEEE
 #include "mp_kernel.cuh"
 #include "mp_launch.h"

@@ -12,9 +12,12 @@
 //    capacities, thicknesses, humidities), so a reciprocal is the hardware's
 //    approximation and one step of the cubic Newton iteration
 //    r' = r + r (e + e^2), e = 1 - b r, and a quotient is Markstein's
-//    q + (a - b q) r (IBM J. Res. Dev. 34, 1990): the correctly rounded
-//    quotient (none of 1.2e9 random ones differed); a divisor used several
-//    times shares its reciprocal;
+//    q + (a - b q) r (IBM J. Res. Dev. 34, 1990). A zero, infinite or
+//    subnormal divisor gives a NaN. The quotient is the correctly rounded one
+//    but for some that lie within 1e-15 units of a midpoint between two numbers
+//    (none of 4e7 random operands, 14 of 5e6 made to lie there); in a
+//    SHIELD_IEEE unit it is for all. A divisor used several times shares its
+//    reciprocal;
 //  * square roots of values >= 0 by Goldschmidt's coupled iteration on the
 //    hardware's reciprocal square root, with the residual x - g^2 taken
 //    exactly at the end (2 of 1.2e9 differed from the rounded root);
@@ -24,8 +27,8 @@
 //    argument out of their range takes CUDA's function. A power keeps its
 //    exponent in two parts and loses less than exp(c log x) does.
 // A unit that defines SHIELD_IEEE keeps the rounding of every operation of
-// the reference's expressions (CUDA's exp, log, pow and square root, the
-// quotients above): see mp_ieee.cu. On the host (the adjoint tests' harness)
+// the reference's expressions (CUDA's exp, log, pow and square root, quotients as
+// IEEE division rounds them): see mp_ieee.cu. On the host (the adjoint tests' harness)
 // and for any type but double the names are the plain operators and library
 // functions.
 #pragma once
@@ -78,14 +81,25 @@ SHP double qmax(double a, double b) { return a >= b ? a : b; }
 
 // ---------------------------------------------------------------- division
 #ifdef __CUDACC__
-// 1 / b of a finite, normal b
+// 1 / b of a finite, normal b, within one unit in the last place. e + e^2
+// rounds up, so that a b of all ones gets the upper of the two numbers its
+// reciprocal lies between (1 / (2 - 2^-52) = 1/2 + 2^-54 + 2^-107, just above
+// their midpoint; rounded to nearest, e + e^2 would lose the last term).
+// With SHIELD_IEEE one Newton step more gives the correctly rounded 1 / b:
+// from within a unit it does for every other b (Markstein 1990).
 __device__ __forceinline__ double recip(double b) {
   double r;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(b));
   const double e = __fma_rn(-b, r, 1.0);
-  return __fma_rn(r, __fma_rn(e, e, e), r);
+  r = __fma_rn(r, __fma_ru(e, e, e), r);
+#ifdef SHIELD_IEEE
+  r = __fma_rn(r, __fma_rn(-b, r, 1.0), r);
+#endif
+  return r;
 }
-// a / b given r = recip(b)
+// a / b given r = recip(b), for a normal quotient. With r correctly rounded,
+// so is the quotient: its residual a - b q is exact, and r's error moves it
+// by less than a quotient's distance from the nearest midpoint.
 __device__ __forceinline__ double quot(double a, double b, double r) {
   const double q = __dmul_rn(a, r);
   return __fma_rn(__fma_rn(-b, q, a), r, q);
