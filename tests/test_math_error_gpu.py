@@ -1,0 +1,44 @@
+"""The device's exponential, logarithm, powers and saturation humidities lose
+no more than the functions they replace (CUDA's exp, log and pow, and the
+reference's expressions of them): over each range of arguments that the step
+meets, against extended precision, neither the largest error nor the mean
+square exceeds CUDA's on the same arguments.
+
+A result within 0.51 units in the last place counts as correctly rounded, and
+mean squares that differ by less than 0.2 % as equal: a correctly rounded
+result has 0.5 and 0.2887 units by itself, and two such functions differ by
+that much over a million arguments (the mean square of N uniform errors
+scatters by 0.9 / sqrt(N))."""
+import numpy as np
+import pytest
+
+from test_math_gpu import EXP, LD, device, ulps
+
+pytestmark = pytest.mark.gpu
+
+CUDA_EXP = 9
+N = 1_000_000
+
+
+def mantissas(rng, lo, hi):
+    """Numbers between lo and hi, uniform in each binade. (Exponentials of
+    uniform numbers would have logarithms next to doubles.)"""
+    x = np.ldexp(rng.uniform(1.0, 2.0, N), rng.integers(np.floor(np.log2(lo)), np.ceil(np.log2(hi)), N))
+    return x[(x >= lo) & (x <= hi)]
+
+
+def compare(fn, cuda, x, y, exact, what):
+    stats = []
+    for f in (fn, cuda):
+        u = ulps(device(f, x, y), exact).astype(float)
+        stats.append((u.max(), np.sqrt(np.mean(u**2))))
+    (worst, rms), (cuda_worst, cuda_rms) = stats
+    print(f"{what}: {worst:.4f} (rms {rms:.4f}), CUDA {cuda_worst:.4f} ({cuda_rms:.4f})")
+    assert worst <= max(0.51, cuda_worst)
+    assert rms <= 1.002 * cuda_rms
+
+
+@pytest.mark.parametrize("lo,hi", [(-0.35, 0.35), (-3.0, 3.0), (-25.0, 5.0), (-60.0, 60.0), (-699.0, 699.0)])
+def test_exp(lo, hi):
+    x = np.random.default_rng(1).uniform(lo, hi, N)
+    compare(EXP, CUDA_EXP, x, None, np.exp(LD(x)), f"exp [{lo}, {hi}]")
