@@ -63,10 +63,10 @@ static __constant__ double EXP2_C[11] = {
     0.693147180559945325805,   0.240226506959101312602,   0.0555041086648200832261,  0.00961812910759412007516,
     0.00133335581467746208208, 0.000154035304571121010251, 0.0000152527334931271240257, 0.000001321543528230637037,
     1.01781995720268829334e-7, 7.0737832484981793467e-9,  4.43477126654816555124e-10};
-// (2 atanh(s) / s - 2) / s^2 in z = s^2, sqrt(1/2) <= m < sqrt(2), s = (m - 1) / (m + 1), degree 6 (2.5e-18 of log m / s)
-static __constant__ double LOG_C[7] = {0.666666666666673441216, 0.399999999994146787147, 0.285714287423875528243,
-                                0.222221985731911054359, 0.181835643258000383417, 0.153140505598382182471,
-                                0.147959496270289403915};
+// (2 atanh(s) / s - 2) / s^2 in z = s^2, sqrt(1/2) <= m < sqrt(2), s = (m - 1) / (m + 1), degree 7 (1.6e-20 of log m / s)
+static __constant__ double LOG_C[8] = {0.666666666666666609796, 0.400000000000062424342, 0.28571428569087348774,
+                                       0.222222226465718982078, 0.181817756837742750264, 0.153870899487081287653,
+                                       0.132501365763733722032, 0.132511596952031750849};
 #endif
 
 // ------------------------------------------------------- minimum and maximum
@@ -236,40 +236,60 @@ __device__ __forceinline__ double fast_exp(double x) {
   if (!(fabs(x) < 700.0)) return exp(x);
   return exp_reduced(x);
 }
-// x = 2^k m, s = (m - 1) / (m + 1): k and 2 atanh(s) = log m. x positive, finite, normal.
-__device__ __forceinline__ double log_reduced(double x, double& kd) {
+// x = 2^k m: k, s = (m - 1) / (m + 1) with sl, the rounding of its quotient
+// and of m + 1, and 2 (atanh(s) - s), which is log m less 2 (s + sl). x
+// positive, finite, normal.
+struct LogParts {
+  double k, s, sl, t;
+};
+__device__ __forceinline__ LogParts log_parts(double x) {
   const int hi = __double2hiint(x);
   const int k = (hi - 0x3fe6a09e) >> 20;  // m in [sqrt(1/2), sqrt(2))
   const double m = __hiloint2double(hi - (k << 20), __double2loint(x));
-  kd = __dadd_rn(__hiloint2double(0x43300000, k ^ 0x80000000), -4503601774854144.0);  // 2^52 + 2^31 + k, less that
   const double f = __dadd_rn(m, -1.0);
-  const double d = __dadd_rn(m, 1.0);
-  const double s = quot(f, d, recip(d));
-  const double z = __dmul_rn(s, s);
+  const double d = __dadd_rn(m, 1.0), dl = __dadd_rn(m, -__dadd_rn(d, -1.0));
+  const double rd = recip(d);
+  LogParts P;
+  P.k = __int2double_rn(k);
+  P.s = __dmul_rn(f, rd);
+  P.sl = __dmul_rn(__fma_rn(-P.s, dl, __fma_rn(-P.s, d, f)), rd);
+  const double z = __fma_rn(__dadd_rn(P.s, P.s), P.sl, __dmul_rn(P.s, P.s));
   const double z2 = __dmul_rn(z, z);
-  double e = __fma_rn(LOG_C[6], z2, LOG_C[4]), o = __fma_rn(LOG_C[5], z2, LOG_C[3]);
+  double e = __fma_rn(LOG_C[6], z2, LOG_C[4]), o = __fma_rn(LOG_C[7], z2, LOG_C[5]);
   e = __fma_rn(e, z2, LOG_C[2]);
-  o = __fma_rn(o, z2, LOG_C[1]);
+  o = __fma_rn(o, z2, LOG_C[3]);
   e = __fma_rn(e, z2, LOG_C[0]);
-  const double p = __fma_rn(o, z, e);
-  return __fma_rn(__dmul_rn(s, z), p, __dadd_rn(s, s));
+  o = __fma_rn(o, z2, LOG_C[1]);
+  P.t = __dmul_rn(__dmul_rn(P.s, z), __fma_rn(o, z, e));
+  return P;
+}
+// log x = h + l, l the rounding of h: k ln 2 is exact in its leading part
+// and no smaller than 2 s, so the sums' roundings are
+__device__ __forceinline__ double log_sum(const LogParts& P, double& l) {
+  const double a = __dmul_rn(P.k, LN2_HI), b = __dadd_rn(P.s, P.s);
+  const double c = __dadd_rn(a, b);
+  const double t = __dadd_rn(__dadd_rn(__dadd_rn(a, -c), b),
+                             __fma_rn(P.k, LN2_LO, __dadd_rn(__dadd_rn(P.sl, P.sl), P.t)));
+  const double h = __dadd_rn(c, t);
+  l = __dadd_rn(__dadd_rn(c, -h), t);
+  return h;
 }
 __device__ __forceinline__ bool log_in_range(double x) {
   return (unsigned)(__double2hiint(x) - 0x00100000) < 0x7fe00000u;  // positive, normal, finite
 }
+// 0.53 units in the last place at most (CUDA's log 0.55, the plain sum 2.0)
 __device__ __forceinline__ double fast_log(double x) {
   if (!log_in_range(x)) return log(x);
-  double k;
-  const double l = log_reduced(x, k);
-  return __fma_rn(k, LN2_HI, __fma_rn(k, LN2_LO, l));
+  double l;
+  return log_sum(log_parts(x), l);
 }
 // x^c, x > 0: 2^(c log2 x). log2 x and its product with c are kept in two
 // parts, so that the power is good to about two units in the last place
 // (exp(c log x) rounds the exponent: up to |c log x| units).
 __device__ __forceinline__ double fast_powc(double x, double c) {
   if (!log_in_range(x)) return pow(x, c);
-  double k;
-  const double l = log_reduced(x, k);
+  const LogParts P = log_parts(x);
+  const double k = P.k, l = __dadd_rn(__dadd_rn(P.s, P.s), __dadd_rn(__dadd_rn(P.sl, P.sl), P.t));
   const double h = __fma_rn(l, 1.44269504088896340736, k);
   const double hl = __fma_rn(l, 1.44269504088896340736, __dadd_rn(k, -h));
   const double y = __dmul_rn(c, h);

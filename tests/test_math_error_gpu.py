@@ -12,11 +12,11 @@ scatters by 0.9 / sqrt(N))."""
 import numpy as np
 import pytest
 
-from test_math_gpu import EXP, LD, device, ulps
+from test_math_gpu import EXP, LD, LOG, device, ulps
 
 pytestmark = pytest.mark.gpu
 
-CUDA_EXP = 9
+CUDA_EXP, CUDA_LOG = 9, 10
 N = 1_000_000
 
 
@@ -42,3 +42,9 @@ def compare(fn, cuda, x, y, exact, what):
 def test_exp(lo, hi):
     x = np.random.default_rng(1).uniform(lo, hi, N)
     compare(EXP, CUDA_EXP, x, None, np.exp(LD(x)), f"exp [{lo}, {hi}]")
+
+
+@pytest.mark.parametrize("lo,hi", [(1e-14, 1.0), (1e-9, 1e-2), (0.5, 2.0), (0.7, 1.42), (0.9, 1.1), (1e-300, 1e300)])
+def test_log(lo, hi):
+    x = mantissas(np.random.default_rng(2), lo, hi)
+    compare(LOG, CUDA_LOG, x, None, np.log(LD(x)), f"log [{lo}, {hi}]")
