@@ -15,7 +15,7 @@ using namespace shield;
 enum {
   F_DIV = 0, F_SQRT, F_EXP, F_LOG, F_POW, F_QSW, F_QSW_DT, F_QSI, F_QSI_DT,
   // CUDA's functions and the reference's expressions on them, which the forms above replace
-  G_EXP, G_LOG, G_POW, G_QSW, G_QSW_DT, G_QSI, G_QSI_DT
+  G_EXP, G_LOG, G_POW, G_QSW, G_QSW_DT, G_QSI, G_QSI_DT, G_EXP_LOG
 };
 
 // wqs1 and iqs2 (microphysics_funcs.py:52-145) as the reference writes them
@@ -60,6 +60,7 @@ __global__ void math_kernel(int fn, int n, const double* x, const double* y, dou
     case G_QSW_DT: r = wqs_cuda(K, a, b) * (K.DC_VAP + K.LV0 / a) / (K.RVGAS * a); break;
     case G_QSI: r = iqs_cuda(K, a, b, d); break;
     case G_QSI_DT: iqs_cuda(K, a, b, d), r = d; break;
+    case G_EXP_LOG: r = exp(b * log(a)); break;
   }
   out[i] = r;
 }
@@ -68,13 +69,14 @@ __global__ void math_kernel(int fn, int n, const double* x, const double* y, dou
 
 // out[i] = function `fn` of (x[i], y[i]) for n elements on `stream`: a / b,
 // sqrt, exp, log, x^y, then wqs1, its derivative, iqs1, its derivative at
-// temperature x and density y; then CUDA's exp, log and pow, and the
-// saturation humidities as the reference's expressions of them.
+// temperature x and density y; then CUDA's exp, log and pow, the
+// saturation humidities as the reference's expressions of them, and
+// exp(y log x).
 #ifndef PROBE_MATH
 #define PROBE_MATH shield_probe_math
 #endif
 extern "C" int PROBE_MATH(int fn, int n, const double* x, const double* y, double* out, void* stream) {
-  if (fn < F_DIV || fn > G_QSI_DT || n < 1 || !x || !y || !out) return -1;
+  if (fn < F_DIV || fn > G_EXP_LOG || n < 1 || !x || !y || !out) return -1;
   ShieldMpConfig cfg;
   std::memset(&cfg, 0, sizeof(cfg));
   MpConst K;

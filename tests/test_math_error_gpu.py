@@ -12,11 +12,11 @@ scatters by 0.9 / sqrt(N))."""
 import numpy as np
 import pytest
 
-from test_math_gpu import EXP, LD, LOG, device, ulps
+from test_math_gpu import EXP, LD, LOG, POW, device, ulps
 
 pytestmark = pytest.mark.gpu
 
-CUDA_EXP, CUDA_LOG = 9, 10
+CUDA_EXP, CUDA_LOG, CUDA_POW, CUDA_EXP_LOG = 9, 10, 11, 16
 N = 1_000_000
 
 
@@ -48,3 +48,15 @@ def test_exp(lo, hi):
 def test_log(lo, hi):
     x = mantissas(np.random.default_rng(2), lo, hi)
     compare(LOG, CUDA_LOG, x, None, np.log(LD(x)), f"log [{lo}, {hi}]")
+
+
+@pytest.mark.parametrize("c,replaced", [
+    # the reference's powers: density and mixing ratio, air's density, CCN
+    (0.65625, "CUDA_POW"), (0.6875, "CUDA_POW"), (0.25, "CUDA_POW"), (-1.0 / 3.0, "CUDA_POW"),
+    # those it writes as exp(c log x)
+    (0.0625, "CUDA_EXP_LOG"), (0.2, "CUDA_EXP_LOG"), (0.65625, "CUDA_EXP_LOG"), (0.725, "CUDA_EXP_LOG"),
+    (0.8125, "CUDA_EXP_LOG"), (0.875, "CUDA_EXP_LOG"), (0.95, "CUDA_EXP_LOG"), (1.75, "CUDA_EXP_LOG"),
+    (7.0 / 3.0, "CUDA_EXP_LOG")])
+def test_power(c, replaced):
+    x = mantissas(np.random.default_rng(3), 1e-14, 1e10 if c < 0.0 else 10.0)
+    compare(POW, globals()[replaced], x, c, np.power(LD(x), LD(c)), f"power {c:.4f}")
