@@ -12,11 +12,12 @@ scatters by 0.9 / sqrt(N))."""
 import numpy as np
 import pytest
 
-from test_math_gpu import EXP, LD, LOG, POW, device, ulps
+from test_math_gpu import EXP, LD, LOG, POW, QSI, QSI_DT, QSW, QSW_DT, device, ulps
 
 pytestmark = pytest.mark.gpu
 
 CUDA_EXP, CUDA_LOG, CUDA_POW, CUDA_EXP_LOG = 9, 10, 11, 16
+CUDA_QS = {QSW: 12, QSW_DT: 13, QSI: 14, QSI_DT: 15}
 N = 1_000_000
 
 
@@ -60,3 +61,26 @@ def test_log(lo, hi):
 def test_power(c, replaced):
     x = mantissas(np.random.default_rng(3), 1e-14, 1e10 if c < 0.0 else 10.0)
     compare(POW, globals()[replaced], x, c, np.power(LD(x), LD(c)), f"power {c:.4f}")
+
+
+@pytest.mark.parametrize("ice", [False, True])
+@pytest.mark.parametrize("lo,hi", [(170.0, 330.0), (200.0, 273.15), (273.2, 310.0), (150.1, 398.9)])
+def test_saturation_humidity(lo, hi, ice):
+    from pyshield_b200 import constants as C
+
+    rng = np.random.default_rng(4)
+    t, den = rng.uniform(lo, hi, N), np.exp(rng.uniform(np.log(1e-3), np.log(2.0), N))
+    cold = ice & (t < C.TICE)
+    dc, lh = np.where(cold, LD(C.D2ICE), LD(C.DC_VAP)), np.where(cold, LD(C.LI2), LD(C.LV0))
+    t0, rv = LD(C.TICE), LD(C.RVGAS)
+    te = np.minimum(LD(t), t0 + 102) if ice else LD(t)
+    q = LD(C.E00) * np.exp((dc * np.log(te / t0) + lh * (te - t0) / (te * t0)) / rv) / (rv * te * LD(den))
+    for fn, exact in ((QSI if ice else QSW, q), (QSI_DT if ice else QSW_DT, q * (dc + lh / te) / (rv * te))):
+        stats = []
+        for f in (fn, CUDA_QS[fn]):
+            err = np.abs(LD(device(f, t, den)) / exact - 1).astype(float)
+            stats.append((err.max(), np.sqrt(np.mean(err**2))))
+        (worst, rms), (ref_worst, ref_rms) = stats
+        print(f"{'ice' if ice else 'water'} {fn} [{lo}, {hi}]: {worst:.2e} ({rms:.2e}), "
+              f"reference {ref_worst:.2e} ({ref_rms:.2e})")
+        assert worst <= ref_worst and rms <= ref_rms
