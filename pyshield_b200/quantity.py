@@ -9,6 +9,7 @@ element strides are passed to the kernels.
 """
 
 import struct
+from operator import index
 
 import numpy as np
 
@@ -72,7 +73,7 @@ def _unpack(q):
     ptr, strides, shape = _array_info(data)
     if origin is None:
         origin = (0,) * len(shape)
-    return ptr, strides, shape, tuple(origin)
+    return ptr, strides, shape, tuple(map(index, origin))
 
 
 def field3d(q, extent=None):
@@ -115,7 +116,8 @@ def _words3d(qs, ext):
             continue
         si, sj, sk = data.stride()
         ni, nj, nk = data.shape
-        oi, oj, ok = getattr(q, "origin", None) or (0, 0, 0)
+        org = getattr(q, "origin", None)
+        oi, oj, ok = (0, 0, 0) if org is None else tuple(org)[:3]
         if oi < 0 or oj < 0 or ok < 0 or oi + nx > ni or oj + ny > nj or ok + nz > nk:
             raise ValueError(f"domain origin {(oi, oj, ok)} extent {tuple(ext)} exceeds storage {(ni, nj, nk)}")
         out += (data.data_ptr() + 8 * (oi * si + oj * sj + ok * sk), si, sj, sk)
