@@ -216,10 +216,10 @@ class Physics:
         self._dm3d = quantity_factory.zeros([X_DIM, Y_DIM, Z_DIM], "unknown")
         self._del_gz = quantity_factory.zeros([X_DIM, Y_DIM, Z_DIM], "unknown")
         self._gfs_microphysics = "GFS_microphysics" in schemes
-        self._de_ice = bool(namelist.de_ice)
         if self._gfs_microphysics:
             self._microphysics = Microphysics(stencil_factory, quantity_factory, grid_data, namelist,
                                               precision=precision)
+            self._de_ice = bool(namelist.de_ice)
         self._fields = ShieldPhysicsFields()
         load()
 
