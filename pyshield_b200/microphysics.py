@@ -152,6 +152,9 @@ class Microphysics:
         whole and their contents are not read (what zeroing them and
         ``__call__`` leave). Not with ``de_ice``, which reads ``qi_dt``."""
         self._build_fields(state)
+        self._launch_fresh(timestep, stream)
+
+    def _launch_fresh(self, timestep, stream=None):
         rc = load().shield_mp_step_fresh(
             self._handle, ctypes.byref(self._fields), float(timestep), _PRECISION[self.precision],
             ctypes.c_void_p(_current_stream(stream)),

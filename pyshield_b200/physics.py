@@ -313,9 +313,16 @@ class Physics:
         # (2.60 ms): the step's blocks are eight columns wide, and ten more
         # 64-byte write streams cost it more than the update's own launch.
         fresh = m is not None and not self._de_ice
+        if fresh:
+            # the tendencies are refused here, as the pre-step that zeroes
+            # them would, and not once it has changed the state
+            self._microphysics._build_fields(m)
         self._prestep(ps, stream, dycore_state, zero_tendencies=not fresh)
         if m is not None:
-            (self._microphysics.step_fresh if fresh else self._microphysics)(m, timestep, stream=stream)
+            if fresh:
+                self._microphysics._launch_fresh(timestep, stream)
+            else:
+                self._microphysics(m, timestep, stream=stream)
             update_physics_state_with_tendencies(
                 ps.qvapor, ps.qliquid, ps.qrain, ps.qice, ps.qsnow, ps.qgraupel, ps.qcld, ps.pt, ps.ua, ps.va,
                 m.qv_dt, m.ql_dt, m.qr_dt, m.qi_dt, m.qs_dt, m.qg_dt, m.qa_dt, m.pt_dt, m.udt, m.vdt,
