@@ -47,7 +47,7 @@ struct Column {
   static constexpr int WP = Tiles<NW>::RP;  // pitch of the work rows
   int w, lane, k, L, bar;
   static constexpr int CV = 10;     // doubles of the column's own values
-  static constexpr int NPARK = 13;  // doubles of a thread's slot (ParkSlot)
+  static constexpr int NPARK = 13;  // doubles of a thread's slot (ParkSlot, and one to make it odd)
   double* scr;   // 2 * SCR doubles
   double* work;  // 2 * RP doubles, for the sequential vapour borrow: the threads' slots, before they are used
   double* park;  // this thread's slot
@@ -80,31 +80,6 @@ struct Column {
     sync();
     if (lane == 0 && w > 0) u = s[w - 1];
     return u;
-  }
-  SHD void prev2(double x, double y, double& px, double& py) {
-    px = __shfl_up_sync(FULLMASK, x, 1);
-    py = __shfl_up_sync(FULLMASK, y, 1);
-    if (NW == 1) return;
-    double* s = slot();
-    if (lane == 31) {
-      s[2 * w] = x;
-      s[2 * w + 1] = y;
-    }
-    sync();
-    if (lane == 0 && w > 0) {
-      px = s[2 * w - 2];
-      py = s[2 * w - 1];
-    }
-  }
-  // value at level k + 1 (undefined at k = 32 NW - 1)
-  SHD double next(double x) {
-    double d = __shfl_down_sync(FULLMASK, x, 1);
-    if (NW == 1) return d;
-    double* s = slot();
-    if (lane == 0) s[w] = x;
-    sync();
-    if (lane == 31 && w < NW - 1) d = s[w + 1];
-    return d;
   }
   SHD bool any(bool p) {
     if (NW == 1) return __any_sync(FULLMASK, p);
@@ -254,11 +229,6 @@ struct Column {
     sync();
     x0 = s[0];
     y0 = s[1];
-  }
-  SHD double bcast(double x, int k0) {
-    double x0, y0;
-    bcast2(x, x, k0, x0, y0);
-    return x0;
   }
   // X_k = a_k + b_k X_{k-1} from the top down (b must vanish at k = 0)
   SHD double scan_affine(double a, double b) {
@@ -417,22 +387,6 @@ struct Column {
       x[n] = A[n] + B[n] * X;
     }
   }
-  // values of N fields at level k0 with one barrier
-  template <int N>
-  SHD void bcastN(const double (&x)[N], int k0, double (&x0)[N]) {
-    const int w0 = k0 >> 5, l0 = k0 & 31;
-#pragma unroll
-    for (int n = 0; n < N; ++n) x0[n] = __shfl_sync(FULLMASK, x[n], l0);
-    if (NW == 1) return;
-    double* s = slot();
-    if (w == w0 && lane == 0) {
-#pragma unroll
-      for (int n = 0; n < N; ++n) s[n] = x0[n];
-    }
-    sync();
-#pragma unroll
-    for (int n = 0; n < N; ++n) x0[n] = s[n];
-  }
   // layer thickness from the BACKWARD height sweep with one barrier:
   // ze_k = zs + sum_{j >= k} (-dz1_j); dz_k = ze_k - ze_{k+1}, dz_{L-1} = ze_{L-1} - zs
   SHD double heights(double t, double zs) {
@@ -481,18 +435,6 @@ struct Column {
 #pragma unroll
       for (int n = 0; n < N; ++n) xn[n] = s[N * (w + 1) + n];
     }
-  }
-  // x at level k - 1 and y at level k + 1 with one barrier
-  SHD void prev_next(double x, double y, double& xp, double& yn) {
-    xp = __shfl_up_sync(FULLMASK, x, 1);
-    yn = __shfl_down_sync(FULLMASK, y, 1);
-    if (NW == 1) return;
-    double* s = slot();
-    if (lane == 31) s[2 * w] = x;
-    if (lane == 0) s[2 * w + 1] = y;
-    sync();
-    if (lane == 0 && w > 0) xp = s[2 * (w - 1)];
-    if (lane == 31 && w < NW - 1) yn = s[2 * (w + 1) + 1];
   }
   // N independent bottom-up affine scans X_k = a_k + c_k X_{k+1} with one
   // barrier (c must vanish at the last level); the adjoints of the
@@ -556,21 +498,6 @@ struct Column {
     for (int u = 1; u < NW; ++u) t = t + s[u];
     return t;
   }
-  // inclusive sum from the bottom: sum over levels j >= k
-  SHD double suffix_sum(double t) {
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-      double v = __shfl_down_sync(FULLMASK, t, d);
-      if (lane + d < 32) t = t + v;
-    }
-    if (NW == 1) return t;
-    double* s = slot();
-    if (lane == 0) s[w] = t;
-    sync();
-    double c = 0.0;
-    for (int u = NW - 1; u > w; --u) c = c + s[u];
-    return t + c;
-  }
 };
 
 // P columns of L levels packed one after another on the 32 NWG threads of
@@ -601,7 +528,7 @@ struct PackedColumn {
   int wf;      // first warp of this thread's column
   int off;     // 1: the column starts inside that warp
   static constexpr int CV = 10;     // doubles of a column's own values
-  static constexpr int NPARK = 13;  // doubles of a thread's slot (ParkSlot)
+  static constexpr int NPARK = 13;  // doubles of a thread's slot (ParkSlot, and one to make it odd)
   static_assert((P + 1) * 2 * WP <= T * NPARK, "the work rows lie in the threads' slots");
   double* scr;   // 2 * SCR doubles
   double* work;  // this column's two work rows (WP doubles each), in the threads' slots before they are used
@@ -668,14 +595,6 @@ struct PackedColumn {
   // ------------------------------------------------ neighbour exchanges
   // (values of another column, read at a column's ends, are not used by
   // the callers, which select the boundary value at k = 0 / k = L - 1)
-  SHD double prev(double x) {
-    double u = __shfl_up_sync(FULLMASK, x, 1);
-    double* s = slot();
-    if (lane() == 31) s[w()] = x;
-    sync();
-    if (lane() == 0 && w() > 0) u = s[w() - 1];
-    return u;
-  }
   template <int N>
   SHD void nbrsN(const double (&x)[N], double (&xp)[N], double (&xn)[N]) {
     double* s = slot();
@@ -1178,7 +1097,7 @@ struct StepGeom {
 // takes the same time alone on an SM as with three others: 33 against 42 us
 // at L79), and registers decide those: the state in use stays in registers,
 // these values are read where they are needed.
-enum ParkSlot { PK_W, PK_DP1, PK_P1, PK_DZ, PK_DZ1, PK_DENFAC, PK_M1, PK_MP, PK_M1SOL, PK_MPSOL, PK_VTR, PK_VTG, PK_VTS };
+enum ParkSlot { PK_W, PK_DP1, PK_P1, PK_DZ, PK_DZ1, PK_DENFAC, PK_MP, PK_M1SOL, PK_MPSOL, PK_VTR, PK_VTG, PK_VTS };
 struct LevelStore {
   double* pk;  // this thread's slot
   double* cv;  // the column's values: fields_init's, written by level 0 and read after the next exchange (or order())
@@ -1189,9 +1108,8 @@ struct LevelStore {
   SHD double& dz() const { return pk[PK_DZ]; }    // start of each sub-step
   SHD double& dz1() const { return pk[PK_DZ1]; }
   SHD double& denfac() const { return pk[PK_DENFAC]; }
-  // the precipitation flux summed over the sub-steps, here and at the level
-  // above; the solid flux of the last sedimentation likewise
-  SHD double& m1() const { return pk[PK_M1]; }
+  // the precipitation flux at the level above, summed over the sub-steps; the
+  // solid flux of the last sedimentation, here (kept by a recorder) and there
   SHD double& mp() const { return pk[PK_MP]; }
   SHD double& m1_sol() const { return pk[PK_M1SOL]; }
   SHD double& mp_sol() const { return pk[PK_MPSOL]; }
@@ -1301,7 +1219,6 @@ SHD void fields_init(Col& C, const MpConst& K, bool valid, double pt, double qvi
   P.w() = wz;
   P.dp1() = dp1;
   P.p1() = p1;
-  P.m1() = 0.0;
   P.mp() = 0.0;
 }
 
@@ -1412,8 +1329,8 @@ SHD void warm_rain(Col& C, const MpConst& K, const MpConstF& KF, bool valid, Lev
 
 // sedimentation (:657-1217): fall speeds, cloud ice melting, and the
 // implicit falls of ice, snow and graupel with their vertical-velocity
-// transport and heating. Stores the solid flux at this level and at the level
-// above; the bottom level adds the surface fluxes to the column's totals. A
+// transport and heating. Stores the solid flux at the level above (with a
+// recorder, here too); the bottom level adds the surface fluxes to the column's totals. A
 // recorder gets the cloud ice fall speed (value 0).
 template <bool MIXED, class Col, class Rec = NoRec>
 SHD void sedimentation(Col& C, const MpConst& K, const MpConstF& KF, bool valid, LevState& S,
@@ -1501,7 +1418,7 @@ SHD void sedimentation(Col& C, const MpConst& K, const MpConstF& KF, bool valid,
     if (bottom) C.cv[CV_GRAUPEL] += flux[2];
   }
   P.w() = w;
-  P.m1_sol() = m1_sol;
+  if constexpr (Rec::on) P.m1_sol() = m1_sol;
   P.mp_sol() = m1_prev;
   if constexpr (Rec::on) S.w = w;
   if (K.do_sedi_heat) sedi_heat(C, K, tz, P.dz1(), dp1, qv, ql, qr, qi, qs, qg, m1_sol, m1_prev, valid, K.C_ICE);
@@ -1597,7 +1514,6 @@ SHD void mp_body(const MpArgs& A, double* sm, double* scr, double* work, const i
       warm_rain<MIXED>(C, K, KF, valid, S, P, m1_rain, mp_rain, FLAGS ? &falls : nullptr);
       if constexpr (FLAGS) fl |= falls ? (is_first ? FLAG_RAIN_FALLS_1 : FLAG_RAIN_FALLS_2) : 0u;
       if (k == L - 1) C.cv[CV_RAIN] += m1_rain;
-      P.m1() = is_first ? P.m1() + m1_rain : P.m1() + m1_rain + P.m1_sol();
       P.mp() = is_first ? P.mp() + mp_rain : P.mp() + mp_rain + P.mp_sol();
       if (!is_first) break;
       sedimentation<MIXED>(C, K, KF, valid, S, P, FLAGS ? &fl : nullptr);
