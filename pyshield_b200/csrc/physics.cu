@@ -110,7 +110,7 @@ constexpr int TC = 32;
 constexpr int NWB = 16;
 
 template <bool FUSED, bool SAME>
-__global__ void __launch_bounds__(TC * NWB, FUSED ? 1 : PRE_MINB)
+__global__ void __launch_bounds__(TC * NWB, FUSED || !SAME ? 1 : PRE_MINB)
     physics_prestep_kernel(const __grid_constant__ PhysArgs A) {
   extern __shared__ double smem[];
   const int nxf = A.nx + 2 * A.hx;
