@@ -51,15 +51,15 @@ HALO = 3
 
 # DRAM bytes (read + write) per algorithmic byte of the step kernel, from an
 # ncu capture of the C48 L79 workload (dram__bytes_read.sum +
-# dram__bytes_write.sum = 239.23 + 76.23 MB for 315.19 MB of algorithmic
+# dram__bytes_write.sum = 239.23 + 75.66 MB for 315.19 MB of algorithmic
 # traffic); the kernel streams each field once, so the ratio carries over
 # to C96.
-NCU_TRAFFIC_RATIO = (239.227648 + 76.229376) / 315.19
+NCU_TRAFFIC_RATIO = (239.230464 + 75.661056) / 315.19
 
 # FP64 flops per column-step of the plain step kernel (2 per DFMA, 1 per
 # DADD or DMUL, thread-level counts of predicated-on instructions), from an
 # ncu capture of the C48 launch divided by its columns; by level count.
-FP64_FLOPS_PER_COLUMN_STEP = {79: (2 * 816161944 + 422208009 + 619919400) / 13824}
+FP64_FLOPS_PER_COLUMN_STEP = {79: (2 * 866476494 + 500262058 + 615596237) / 13824}
 
 
 def algorithmic_bytes_per_column_step(nlev):

@@ -78,7 +78,13 @@ def step_forward(mp, state, land, timestep, stream=None, tendencies=None):
     ``tendencies`` (dict of tendency name -> field, missing ones zero): the
     incoming tendencies the step adds its increments to, which the outputs
     then include; with ``de_ice`` the step reads ``qi_dt`` and rewrites
-    ``qi_dt``, ``qs_dt``, qice and qsnow (state copies are used here)."""
+    ``qi_dt``, ``qs_dt``, qice and qsnow (state copies are used here).
+
+    The plain FP64 step with the rounding of every operation of the
+    reference's expressions (``shield_mp_step_ieee``): the outputs agree with
+    ``Microphysics.__call__``'s to round-off, not to the bit. Over a window,
+    branches hang on the sign of rounding residues, and the adjoint takes
+    them as this forward does."""
     import torch
 
     _check_state(mp, state)
@@ -159,7 +165,8 @@ try:
     class MicrophysicsStep(torch.autograd.Function):
         """``outputs = MicrophysicsStep.apply(mp, timestep, land, *state)``:
         the 16 outputs (``OUTPUTS``) of one step of ``mp`` from its 14
-        inputs (``STATE``); differentiable in every input."""
+        inputs (``STATE``), as ``step_forward`` gives them; differentiable in
+        every input."""
 
         @staticmethod
         def forward(ctx, mp, timestep, land, *state):

@@ -127,6 +127,11 @@ struct AtmArgs {
 // 2 blocks 0.324 / 0.642 / 0.054; 128 x 8, one block 0.370. More warps give
 // each phase more loads in flight; beyond 32 a SM the registers spill (48
 // warps 0.406). Without phases 4 and 5 the launch takes 0.288.
+// Phase 2 by need (C96 L79 / L127): 0.286 / 0.437 where no level of any column
+// needs it, 0.329 / 0.546 with needy halo columns alone (a third of the blocks),
+// 0.326 / 0.499 with 1 % of the levels needy and 0.335 / 0.507 with every other
+// one, both sweeps in every block; always swept, with an offset per field and
+// 4 level warps, 0.384 to 0.400 / 0.730 to 0.751.
 constexpr int AT_TC = 32, AT_LW = 16, AT_MINB = 2;
 
 template <bool SAME>

@@ -1712,7 +1712,10 @@ using Packed80 = PackedLayout<5, 2, 4>;
 // 8: 2.06 / 1.52, 9: 2.19 / 1.55; L127 4: 3.51 / 2.55, 5: 3.30 / 2.36,
 // 6: 3.22 / 2.27, 7 (28 warps, 72 registers): 3.16 / 2.19, 8: 3.40 / 2.33.
 // At L127 the 7-column block is the faster one only when its waves are many
-// (3,233 columns, 4 waves of either: 0.226 against 0.205).
+// (3,233 columns, 4 waves of either: 0.226 against 0.205). These times compare
+// the shapes, with the arithmetic of the day; the shapes taken now run L31 in
+// 0.71 / 0.50, L63 1.54 / 1.11, L79 1.87 / 1.39, L90 2.01 / 1.55 and L127
+// 3.10 / 2.22.
 template <bool MIXED, bool FLAGS>
 cudaError_t launch_shapes(const MpArgs& A, cudaStream_t st) {
   const int L = A.nz;

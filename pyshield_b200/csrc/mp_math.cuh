@@ -4,10 +4,13 @@
 // The step meets about 200 divisions and square roots and 50 exponentials
 // and logarithms per level. With the general forms, most of the step's
 // instructions were not its arithmetic but theirs: range checks, branches to
-// a slow path, 64-bit literal coefficients built in pairs of moves (ncu,
-// C48 L79: 490 M warp instructions, 140 M of them FP64; now 307 M and 102 M,
-// and the C96 L79 step 3.61 -> 2.14 ms, mixed 2.29 -> 1.63 ms). The forms
-// here drop what the step's operands do not need:
+// a slow path, 64-bit literal coefficients built in pairs of moves (ncu, C48
+// L79: 490 M warp instructions, 140 M of them FP64; with these forms, when
+// they came in, 307 M and 102 M, and the C96 L79 step 3.61 -> 2.14 ms, mixed
+// 2.29 -> 1.63 ms). Exp, log, powers and the humidity over ice were less
+// accurate than the functions replaced then; carrying the roundings that
+// mends it took 1.82 -> 1.87 ms, mixed 1.38 -> 1.39. The forms here drop what
+// the step's operands do not need:
 //  * divisors are finite and normal (temperatures, densities, heat
 //    capacities, thicknesses, humidities), so a reciprocal is the hardware's
 //    approximation and one step of the cubic Newton iteration

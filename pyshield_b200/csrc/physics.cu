@@ -105,6 +105,10 @@ __device__ __forceinline__ double np_min(double a, double b) { return a <= b ? a
 // tendencies): 8, 2 with an offset per field 0.502; one offset and 8, 2
 // 0.499; 16, 2 (64 registers) 0.475. Without the zeroing (Physics.__call__,
 // whose step writes the tendencies anew) 0.310.
+// An offset per field does not fit 64 registers: those forms, and the fused
+// one, take one block per SM (k-fastest storages, 12 x 12 / 53 x 61 / C96
+// columns of L79: 0.088 / 0.111 / 1.302 with two, 0.068 / 0.090 / 1.197 with
+// one; 8 warps, 2 blocks 0.070 / 0.101 / 1.405).
 constexpr int PRE_MINB = 2;
 constexpr int TC = 32;
 constexpr int NWB = 16;
