@@ -73,7 +73,7 @@ def _unpack(q):
     ptr, strides, shape = _array_info(data)
     if origin is None:
         origin = (0,) * len(shape)
-    return ptr, strides, shape, tuple(map(index, origin))
+    return ptr, strides, shape, tuple(origin)
 
 
 def field3d(q, extent=None):
@@ -85,7 +85,7 @@ def field3d(q, extent=None):
     for d in range(3):
         if org[d] < 0 or org[d] + ext[d] > shape[d]:
             raise ValueError(f"domain origin {org} extent {ext} exceeds storage {shape}")
-    off = org[0] * st[0] + org[1] * st[1] + org[2] * st[2]
+    off = index(org[0] * st[0] + org[1] * st[1] + org[2] * st[2])
     return ShieldField3D(ptr + 8 * off, st[0], st[1], st[2])
 
 
@@ -97,7 +97,7 @@ def field2d(q, extent=None):
     for d in range(2):
         if org[d] < 0 or org[d] + ext[d] > shape[d]:
             raise ValueError(f"domain origin {org} extent {ext} exceeds storage {shape}")
-    off = org[0] * st[0] + org[1] * st[1]
+    off = index(org[0] * st[0] + org[1] * st[1])
     return ShieldField2D(ptr + 8 * off, st[0], st[1])
 
 
@@ -117,7 +117,13 @@ def _words3d(qs, ext):
         si, sj, sk = data.stride()
         ni, nj, nk = data.shape
         org = getattr(q, "origin", None)
-        oi, oj, ok = (0, 0, 0) if org is None else tuple(org)[:3]
+        if org is None:
+            oi = oj = ok = 0
+        else:
+            try:
+                oi, oj, ok = org
+            except ValueError:
+                oi, oj, ok = tuple(org)[:3]
         if oi < 0 or oj < 0 or ok < 0 or oi + nx > ni or oj + ny > nj or ok + nz > nk:
             raise ValueError(f"domain origin {(oi, oj, ok)} extent {tuple(ext)} exceeds storage {(ni, nj, nk)}")
         out += (data.data_ptr() + 8 * (oi * si + oj * sj + ok * sk), si, sj, sk)
